@@ -516,9 +516,9 @@ class Engine:
         together; 10 ring, 6 per CTA, two at a time; 11-13 pair kernel;
         14 spread kernel; 15 automatic in fixed summation order (no pair
         kernel: results independent of the batch); 16 spread kernel over a
-        two-SM cluster (lowest latency).  fp64: 0 automatic (the two-SM
-        cluster kernel up to one ciphertext per SM, else 3); 3
-        L2-direct, 3 per CTA; 4 shared key ring; 16 two-SM cluster."""
+        two-SM cluster (lowest latency).  fp64: 0 automatic (waves of 3 per SM
+        on shape 3, smaller remainders on the one-per-CTA or the two-SM
+        cluster kernel); 3 L2-direct, 3 per CTA; 4 shared key ring; 16 two-SM cluster."""
         self._check(self.lib.tfhe_gpu_set_groups_per_cta(self.ctx, self._form(form), int(groups)),
                     "set_groups_per_cta")
 

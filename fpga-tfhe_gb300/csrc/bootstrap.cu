@@ -114,6 +114,26 @@ __device__ __forceinline__ void round_wrap_pair(cpx<float> z, uint32_t& a0, uint
     a1 = (uint32_t)__float2int_rn(sc.y);
 }
 
+// FP64 conversions by integer operations.  The FP64 unit of this part takes
+// 19 clocks per warp instruction and SM (64 for a warp alone), and conversions
+// to and from double 16, so the integer pipe does them: a normal float (or
+// +0) widened by its bits, and the truncation of the inverse transform's
+// output, whose division by 512 is part of the shift.  Exact, so the same
+// values as (double)f and (int64_t)(z / 512) mod 2^32 for |z / 512| < 2^63.
+// FP64 layer of 456 on the 3-per-CTA kernel: 92.6 -> 87.0 ms.
+__device__ __forceinline__ double widen_float(float f) {
+    const uint32_t b = (uint32_t)__float_as_int(f);
+    const uint32_t hi = (b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + ((1023u - 127u) << 20));
+    return b ? __hiloint2double((int)hi, (int)(b << 29)) : 0.0;
+}
+__device__ __forceinline__ uint32_t trunc_div512(double z) {
+    const uint32_t hi = (uint32_t)__double2hiint(z), lo = (uint32_t)__double2loint(z);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023 - 9;  // exponent of z / 512
+    const uint64_t m = ((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+    const uint32_t v = (uint32_t)(e <= 52 ? m >> (52 - max(e, -1)) : m << min(e - 52, 63));
+    return hi >> 31 ? 0u - v : v;
+}
+
 // Gadget digit of u at `decal` as a transform input: ((u >> decal) & mask) -
 // halfBg.  FP32: the masked digit m < 2^22 ORed into the encoding of the
 // magic constant is the float M + m, and one subtraction of M + halfBg
@@ -124,7 +144,7 @@ __device__ __forceinline__ R digit_value(uint32_t u, int decal, uint32_t mask, i
         return __int_as_float((int32_t)(((u >> decal) & mask) | (uint32_t)kRoundMagicBits)) -
                (kRoundMagic + (float)halfBg);
     } else {
-        return (R)((int)((u >> decal) & mask) - halfBg);
+        return (R)widen_float(digit_value<float>(u, decal, mask, halfBg));
     }
 }
 
@@ -139,14 +159,6 @@ __device__ __forceinline__ cpx<R> digit_pair(uint32_t u0, uint32_t u1, int decal
     } else {
         return {digit_value<R>(u0, decal, mask, halfBg), digit_value<R>(u1, decal, mask, halfBg)};
     }
-}
-
-template <typename R>
-__device__ __forceinline__ int64_t to_int(R v);
-template <>
-__device__ __forceinline__ int64_t to_int<double>(double v) {
-    // reference semantics: int64_t(double) truncates (TorusPolynomial_fft.cpp:40)
-    return __double2ll_rz(v);
 }
 
 // ----------------------------------------------------------------------
@@ -357,7 +369,6 @@ __device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB>& S, Keys& ke
     }
 
     // back to the coefficient domain (j unrolled: out[j] must stay in registers)
-    const R inv = (R)(1.0 / 512.0);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         uint32_t c0[8], c1[8];
@@ -389,8 +400,8 @@ __device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB>& S, Keys& ke
                         if (PARTS == 2 && pt == 0) round_small_pair(z, a0, a1);
                         else round_wrap_pair(z, a0, a1);
                     } else {
-                        a0 = (uint32_t)(uint64_t)to_int<R>(z.x * inv);
-                        a1 = (uint32_t)(uint64_t)to_int<R>(z.y * inv);
+                        a0 = trunc_div512(z.x);  // truncates like the reference (TorusPolynomial_fft.cpp:40)
+                        a1 = trunc_div512(z.y);
                     }
                     if (PARTS == 1) {
                         c0[q] = a0;
@@ -450,11 +461,10 @@ __device__ __forceinline__ void round_part(const cpx<R> (&v)[8], int pt, int spl
             for (int q = 0; q < 8; ++q) round_wrap_pair(v[q], c0[q], c1[q]);
         }
     } else {
-        const R inv = (R)(1.0 / 512.0);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            c0[q] = (uint32_t)(uint64_t)to_int<R>(v[q].x * inv);
-            c1[q] = (uint32_t)(uint64_t)to_int<R>(v[q].y * inv);
+            c0[q] = trunc_div512(v[q].x);
+            c1[q] = trunc_div512(v[q].y);
         }
     }
 }
@@ -1409,6 +1419,131 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
 }
 
 // ----------------------------------------------------------------------
+// The FP64 form's blind rotation, one ciphertext per CTA: 2l groups of 64
+// threads run a step's 2l forward transforms at once, then groups 0 and 1
+// multiply all 2l rows in row order with their output polynomial's part of
+// each key row, transform back and truncate.  The FP64 unit bounds it: 19
+// clocks per warp instruction and SM when all four SM sub-partitions have a
+// warp in FP64 code, 64 when only one has, so the work of a step is laid out
+// to keep all four busy in both halves of it (12 warps, then 4).  A step is
+// about 5,000 FP64 warp instructions, 95,000 clocks (29 ms for n = 630).
+// Measured: 29.8 ms a wave of 152, 59.5 ms for 300, against 43.2 ms (two
+// waves of the cluster kernel) and 92.6 ms (a wave of the 3-per-CTA kernel)
+// before it.
+// The transforms, the products and their order are those of the other FP64
+// shapes.
+// ----------------------------------------------------------------------
+template <int L>
+struct SpreadF64Plan {
+    static constexpr int kGroups = 2 * L;
+    static constexpr size_t acc_off = kHotSize * sizeof(cpx<double>);
+    static constexpr size_t d_off = acc_off + 2 * kN * sizeof(int32_t);            // [row][q][t]
+    static constexpr size_t x_off = d_off + kGroups * kHalf * sizeof(cpx<double>);  // one exchange buffer a group
+    static constexpr size_t total = x_off + kGroups * kScratchStride * sizeof(cpx<double>);
+};
+
+template <int L>
+__global__ void __launch_bounds__(128 * L, 1) k_blind_rotate_spread_f64(KParams kp, Tables T, EpArgs a) {
+    using Plan = SpreadF64Plan<L>;
+    constexpr int kRows = 2 * L;
+    constexpr int kRowElems = 2 * kHalf;  // complex values per key row (two outputs, one part)
+    extern __shared__ __align__(128) char smem[];
+    cpx<double>* tables = reinterpret_cast<cpx<double>*>(smem);
+    int32_t* acc = reinterpret_cast<int32_t*>(smem + Plan::acc_off);
+    cpx<double>* dsh = reinterpret_cast<cpx<double>*>(smem + Plan::d_off);
+    const int c = blockIdx.x;
+    const int g = threadIdx.x >> 6, t = threadIdx.x & 63;
+    const int jp = g / L, lev = g - jp * L;
+    const int n = kp.n;
+    load_hot_tables<double>(tables, T);
+    if (a.acc_in) {
+        const int32_t* src = a.acc_in + (size_t)c * 2 * kN;
+        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x) acc[i] = src[i];
+    } else {
+        const int barb = mod_switch_2n(a.x[(size_t)c * (n + 1) + n]);
+        for (int i = threadIdx.x; i < kN; i += blockDim.x) {
+            acc[i] = 0;
+            acc[kN + i] = test_vector_coef(a, c, barb, i);
+        }
+    }
+    __syncthreads();
+
+    const FftTwiddles<double> tw = hot_twiddles<double>(tables);
+    const FftIdx ix = make_fft_idx(t);
+    cpx<double>* xbuf = reinterpret_cast<cpx<double>*>(smem + Plan::x_off) + g * kScratchStride;
+    const int bar_id = 1 + g;
+    const int halfBg = 1 << (kp.Bgbit - 1);
+    const uint32_t mask = (1u << kp.Bgbit) - 1;
+    const int decal = 32 - (lev + 1) * kp.Bgbit;
+    const cpx<double>* gsw = reinterpret_cast<const cpx<double>*>(a.gsw);
+    const size_t step_elems = (size_t)kRows * kRowElems;
+    const int32_t* bara = a.bara ? a.bara + (size_t)c * n : nullptr;
+    const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
+    const int32_t* rot = bara ? bara : xs;
+    int32_t rot_next = rot[0];
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+        const int ai = bara ? rot_next : mod_switch_2n(rot_next);
+        if (i + 1 < n) rot_next = rot[i + 1];
+        if (ai == 0) continue;  // tfhe_blindRotate_FFT.cpp:114 (uniform over the CTA)
+        const cpx<double>* step_keys = gsw + (size_t)i * step_elems;
+        if (threadIdx.x < kRows)  // this step's rows into L2 during its transforms
+            bulk_prefetch_l2(step_keys + (size_t)threadIdx.x * kRowElems, kRowElems * sizeof(cpx<double>));
+        cpx<double> v[8];
+        {
+            const int32_t* src = acc + jp * kN;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int x0 = t + 64 * q;
+                const uint32_t u0 = (uint32_t)rot_coef(src, x0, ai) - (uint32_t)src[x0] + kp.offset;
+                const uint32_t u1 = (uint32_t)rot_coef(src, x0 + kHalf, ai) - (uint32_t)src[x0 + kHalf] + kp.offset;
+                v[q] = digit_pair<double>(u0, u1, decal, mask, halfBg);
+            }
+        }
+        fft512_forward_ip1(v, xbuf, tw, ix, t, bar_id);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) dsh[(g * 8 + q) * 64 + t] = v[q];
+        __syncthreads();  // every D in place; every read of acc done
+        if (g < 2) {
+            cpx<double> o[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) o[q] = {0.0, 0.0};
+#pragma unroll
+            for (int p = 0; p < kRows; ++p) {
+                const double2* g2 = reinterpret_cast<const double2*>(step_keys + (size_t)p * kRowElems + g * kHalf);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const double2 w = __ldg(g2 + key_index<double>(t, q));
+                    o[q] = cmac(o[q], dsh[(p * 8 + q) * 64 + t], cpx<double>{w.x, w.y});
+                }
+            }
+            fft512_inverse_ip1(o, xbuf, tw, ix, t, bar_id);
+            uint32_t c0[8], c1[8];
+            round_part<double, 1>(o, 0, kp.split, c0, c1);
+            int32_t* dst = acc + g * kN;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int x0 = t + 64 * q;
+                dst[x0] = (int32_t)((uint32_t)dst[x0] + c0[q]);
+                dst[x0 + kHalf] = (int32_t)((uint32_t)dst[x0 + kHalf] + c1[q]);
+            }
+        }
+        __syncthreads();  // the accumulator is updated before the next step reads it
+    }
+    if (a.acc_out) {
+        int32_t* dst = a.acc_out + (size_t)c * 2 * kN;
+        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x) dst[i] = acc[i];
+    }
+    if (a.lwe_out) {
+        // tLweExtractLweSample: a'_0 = a_0, a'_j = -a_{N-j}, b' = b_0
+        int32_t* dst = a.lwe_out + (size_t)c * (kN + 1);
+        for (int i = threadIdx.x; i < kN; i += blockDim.x)
+            dst[i] = i == 0 ? acc[0] : (int32_t)(0u - (uint32_t)acc[kN - i]);
+        if (threadIdx.x == 0) dst[kN] = acc[kN];
+    }
+}
+
+// ----------------------------------------------------------------------
 // Blind rotation with two 64-thread halves per ciphertext (low latency).
 //
 // Half h of a ciphertext decomposes and transforms input polynomial h (rows
@@ -2016,6 +2151,19 @@ cudaError_t launch_spread2_f64(const DevParams& P, const Tables& T, const EpArgs
     return cudaGetLastError();
 }
 
+// FP64: one ciphertext per CTA
+template <int L>
+cudaError_t launch_spread_f64(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
+    if (a.count <= 0) return cudaSuccess;
+    const KParams kp = make_kparams(P);
+    using Plan = SpreadF64Plan<L>;
+    auto kern = k_blind_rotate_spread_f64<L>;
+    cudaError_t e = set_smem(kern, Plan::total);
+    if (e != cudaSuccess) return e;
+    kern<<<a.count, 128 * L, Plan::total, st>>>(kp, T, a);
+    return cudaGetLastError();
+}
+
 // split-FP32 pair kernel with `per_cta` (1..3) ciphertexts per CTA
 template <int L>
 cudaError_t launch_pair_fp32(const DevParams& P, const Tables& T, const EpArgs& a, int per_cta,
@@ -2074,6 +2222,29 @@ cudaError_t launch_auto_fp32(const DevParams& P, const Tables& T, const EpArgs& 
     return launch_spread2<L>(P, T, tail, st);
 }
 
+// Automatic shape of an FP64 blind rotation.  Every shape gives the same
+// ciphertexts, so only time decides.  Measured per launch (default set): the
+// cluster kernel 20.4 ms for up to one ciphertext per two SMs; the
+// one-per-CTA kernel 29.8 ms a wave of one per SM; the 3-per-CTA kernel with
+// L2-direct key reads 87.0 ms a wave of three per SM (3 waves of the former
+// take 89.3 ms).  So whole waves of three per SM, and a remainder of up to
+// two per SM on the one-per-CTA kernel, of up to one per two SMs on the
+// cluster kernel.
+template <int L>
+cudaError_t launch_auto_fp64(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
+    const int wave = 3 * kSmCount;
+    int full = (a.count / wave) * wave;
+    if (a.count - full > 2 * kSmCount) full = a.count;
+    if (full) {
+        const cudaError_t e =
+            launch_ep_t<double, 1, kEpBlindRotate, 3, L>(P, T, slice_blind_rotate(P, a, 0, full), st);
+        if (e != cudaSuccess || full == a.count) return e;
+    }
+    const EpArgs tail = slice_blind_rotate(P, a, full, a.count - full);
+    if (tail.count > kSmCount / 2) return launch_spread_f64<L>(P, T, tail, st);
+    return launch_spread2_f64<L>(P, T, tail, st);
+}
+
 // FP64: ~250 registers per thread and 2 x L exchange buffers of 9 KB per
 // group, so 3 groups (192 threads) per CTA.  split-FP32: GROUPS groups.
 template <int L>
@@ -2084,14 +2255,11 @@ cudaError_t launch_ep_l(const DevParams& P, Form f, EpMode mode, const Tables& T
         case kEpPlain: return launch_ep_t<double, 1, kEpPlain, 3, L>(P, T, a, st);
         case kEpMuxRotate: return launch_ep_t<double, 1, kEpMuxRotate, 3, L>(P, T, a, st);
         default:
-            // 0: automatic -- up to one ciphertext per SM on the cluster
-            // kernel (one or two waves: 21.6 ms each, against about 57 ms for
-            // a wave of the 3-per-CTA kernel), larger batches 3 per CTA with
-            // L2-direct key reads; 3: L2-direct; 4: shared key ring; 16:
-            // cluster kernel
-            if (groups == 16 || (groups == 0 && a.count <= kSmCount))
-                return launch_spread2_f64<L>(P, T, a, st);
-            if (groups == 3 || groups == 0) return launch_ep_t<double, 1, kEpBlindRotate, 3, L>(P, T, a, st);
+            // 0: automatic (launch_auto_fp64); 3: L2-direct, 3 per CTA; 4:
+            // shared key ring; 16: cluster kernel
+            if (groups == 0) return launch_auto_fp64<L>(P, T, a, st);
+            if (groups == 16) return launch_spread2_f64<L>(P, T, a, st);
+            if (groups == 3) return launch_ep_t<double, 1, kEpBlindRotate, 3, L>(P, T, a, st);
             return launch_ring_t<double, 1, 4, L, true>(P, T, a, st);
         }
     }
