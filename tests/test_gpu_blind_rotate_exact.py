@@ -79,3 +79,69 @@ def test_fp64_blind_rotate_from_accumulators(engines, torch_cuda, count):
     bara[:, 5] = 0
     bara[1] = 0
     assert (_rotations(torch, e, "fp64", 0, acc, bara) == _rotations(torch, e, "fp64", 3, acc, bara)).all()
+
+
+def _cur(torch):
+    return torch.cuda.current_stream().cuda_stream
+
+
+def _fft_keys(torch, e, form, count, seed):
+    tgsw = _uniform(torch, seed, count, e.params.tgsw_words())
+    out = torch.empty(count, e.tgsw_fft_bytes(form), device="cuda", dtype=torch.uint8)
+    e.tgsw_to_fft(tgsw, out, count, form, stream=_cur(torch))
+    return out
+
+
+# one item | a few SMs | one more than the SMs | one more than a round of four per SM
+@pytest.mark.parametrize("params,form,count", [("default", "split_fp32", 1), ("stress", "split_fp32", 5),
+                                               ("default", "split_fp32", 153), ("stress", "split_fp32", 609),
+                                               ("default", "fp64", 153), ("stress", "fp64", 457)])
+def test_products_do_not_depend_on_the_batch(engines, torch_cuda, params, form, count):
+    """Item k of a batch of products equals the same item alone, and MuxRotate
+    equals the product of (X^a - 1) acc plus acc (integer identities)."""
+    torch = torch_cuda
+    e = engines(params)
+    gsw = _fft_keys(torch, e, form, count, count)
+    acc = _uniform(torch, count + 1, count, 2048)
+    a = _uniform(torch, count + 2, count) & 2047
+    a[count // 2] = 0
+    got = acc.clone()
+    e.tGswFFTExternMulToTLwe(got, gsw, count, form, stream=_cur(torch))
+    for k in sorted({0, count // 3, count - 1}):
+        one = acc[k:k + 1].clone()
+        e.tGswFFTExternMulToTLwe(one, gsw[k:k + 1], 1, form, stream=_cur(torch))
+        assert torch.equal(one[0], got[k]), k
+    mux = torch.empty_like(acc)
+    e.tfhe_MuxRotate_FFT(mux, acc, gsw, a, count, form, stream=_cur(torch))
+    diff = torch.empty_like(acc)
+    e.tLweMulByXaiMinusOne(diff, a, acc, count, stream=_cur(torch))
+    e.tGswFFTExternMulToTLwe(diff, gsw, count, form, stream=_cur(torch))
+    assert torch.equal(mux, diff + acc)
+    # in place, one TGSW for all
+    e.tfhe_MuxRotate_FFT(mux, acc, gsw, a, count, form, per_item=False, stream=_cur(torch))
+    acc2 = acc.clone()
+    e.tfhe_MuxRotate_FFT(acc2, acc2, gsw, a, count, form, per_item=False, stream=_cur(torch))
+    assert torch.equal(mux, acc2)
+    e.synchronize()
+
+
+@pytest.mark.parametrize("params", ["default", "stress"])
+def test_steps_of_the_blind_rotation_are_the_products(engines, torch_cuda, params):
+    """n MuxRotate calls, one key sample each, give the blind rotation's
+    accumulators bit for bit (split-FP32, key rows summed in order)."""
+    torch = torch_cuda
+    e = engines(params)
+    n, count = e.params.n, 7
+    lwe, tlwe, ks, bk = e.gate_keyset([9])
+    d_bk = torch.from_numpy(bk.reshape(n, -1)).cuda()
+    keys = torch.empty(n, e.tgsw_fft_bytes("split_fp32"), device="cuda", dtype=torch.uint8)
+    e.tgsw_to_fft(d_bk, keys, n, "split_fp32", stream=_cur(torch))
+    acc = _uniform(torch, 21, count, 2048)
+    bara = _uniform(torch, 22, count, n) & 2047
+    want = _rotations(torch, e, "split_fp32", 4, acc, bara)
+    for i in range(n):
+        e.tfhe_MuxRotate_FFT(acc, acc, keys[i], bara[:, i].contiguous(), count, "split_fp32", per_item=False,
+                             stream=_cur(torch))
+    e.synchronize()
+    torch.cuda.synchronize()
+    assert (acc.cpu().numpy() == want).all()
