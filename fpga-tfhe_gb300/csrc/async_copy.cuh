@@ -128,6 +128,12 @@ __device__ __forceinline__ bool mbar_wait_cluster_bounded(uint64_t* bar, uint32_
     return true;
 }
 
+// Order this thread's shared-memory writes before later reads of the async
+// proxy (bulk copies, matrix instructions).
+__device__ __forceinline__ void fence_proxy_async() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // Bulk copy global -> this CTA's shared memory; completion is counted in
 // bytes on `bar`.  dst, src 16-byte aligned; bytes a multiple of 16.
 // Start fetching `bytes` (a multiple of 16, 16-byte aligned) of global

@@ -156,7 +156,7 @@ tfhe_gpu_status run_gates_in(tfhe_gpu_ctx* ctx, const int32_t* gates, int32_t un
     const int split = blind_rotate_tail_start((Form)form, ctx->groups_per_cta[form], count);
     if (split == 0) {
         RET(run_bootstrap_woks(ctx, x, mu, u, count, form, st));
-        CK(ctx, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, u, out, count, st));
+        CK(ctx, launch_keyswitch(ctx->dp, ctx->ks_table(), u, out, count, st));
         return TFHE_GPU_OK;
     }
     // The remainder wave of the blind rotation occupies only part of the
@@ -166,13 +166,13 @@ tfhe_gpu_status run_gates_in(tfhe_gpu_ctx* ctx, const int32_t* gates, int32_t un
     RET(run_bootstrap_woks(ctx, x, mu, u, split, form, st));
     CK(ctx, cudaEventRecord(ctx->ev_fork, st));
     CK(ctx, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-    CK(ctx, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, u, out, split, ctx->side));
+    CK(ctx, launch_keyswitch(ctx->dp, ctx->ks_table(), u, out, split, ctx->side));
     CK(ctx, cudaEventRecord(ctx->ev_join, ctx->side));
     // from here on the caller's stream joins the side stream on every path
     tfhe_gpu_status s = run_bootstrap_woks(ctx, x + (size_t)split * (n + 1), mu, u + (size_t)split * (nk + 1),
                                            count - split, form, st);
     if (s == TFHE_GPU_OK) {
-        const cudaError_t e = launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, u + (size_t)split * (nk + 1),
+        const cudaError_t e = launch_keyswitch(ctx->dp, ctx->ks_table(), u + (size_t)split * (nk + 1),
                                                out + (size_t)split * (n + 1), count - split, st);
         if (e != cudaSuccess) s = cuda_fail(ctx, e, "key switch");
     }
@@ -185,7 +185,7 @@ tfhe_gpu_status run_gates(tfhe_gpu_ctx* ctx, const int32_t* gates, int32_t unifo
                           int32_t* out, const int32_t* ca, const int32_t* cb, int32_t count,
                           int32_t form, cudaStream_t st) {
     RET(need_bk(ctx, form));
-    if (!ctx->d_ks) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     if (count == 0) return TFHE_GPU_OK;
     const int n = ctx->P.n, nk = ctx->P.k * ctx->P.N;
     void *x = nullptr, *u = nullptr;
@@ -277,6 +277,7 @@ void tfhe_gpu_destroy(tfhe_gpu_ctx* ctx) {
     for (int f = 0; f < kNumForms; ++f)
         if (ctx->d_bk[f]) cudaFree(ctx->d_bk[f]);
     if (ctx->d_ks) cudaFree(ctx->d_ks);
+    if (ctx->d_ks_tiles) cudaFree(ctx->d_ks_tiles);
     for (int s = 0; s < 4; ++s)
         if (ctx->d_scratch[s]) cudaFree(ctx->d_scratch[s]);
     if (ctx->d_tables) cudaFree(ctx->d_tables);
@@ -407,7 +408,7 @@ tfhe_gpu_status tfhe_gpu_upload_keyswitch_key(tfhe_gpu_ctx* ctx, const int32_t* 
     const int n = ctx->P.n;
     const int stride = (n + 1 + 3) & ~3;
     const size_t rows = (size_t)ctx->P.k * ctx->P.N * ctx->P.ks_t * (1 << ctx->P.ks_basebit);
-    if (!ctx->d_ks) {
+    if (!ctx->has_ks()) {
         CK(ctx, cudaMalloc(&ctx->d_ks, rows * stride * sizeof(int32_t)));
         ctx->key_bytes += rows * stride * sizeof(int32_t);
     }
@@ -415,6 +416,20 @@ tfhe_gpu_status tfhe_gpu_upload_keyswitch_key(tfhe_gpu_ctx* ctx, const int32_t* 
     CK(ctx, cudaMemset(ctx->d_ks, 0, rows * stride * sizeof(int32_t)));
     CK(ctx, cudaMemcpy2D(ctx->d_ks, stride * sizeof(int32_t), ks, (n + 1) * sizeof(int32_t),
                          (n + 1) * sizeof(int32_t), rows, cudaMemcpyHostToDevice));
+    const size_t tile_bytes = keyswitch_tile_bytes(ctx->dp);
+    if (tile_bytes) {
+        if (!ctx->d_ks_tiles) {
+            CK(ctx, cudaMalloc(&ctx->d_ks_tiles, tile_bytes));
+            ctx->key_bytes += tile_bytes;
+        }
+        CK(ctx, cudaStreamSynchronize(cudaStreamLegacy));  // the rows are in place
+        CK(ctx, launch_keyswitch_tiles(ctx->dp, ctx->d_ks, stride, ctx->d_ks_tiles, ctx->stream));
+        CK(ctx, cudaStreamSynchronize(ctx->stream));
+        // the pieces are the whole table: the rows are not read any more
+        CK(ctx, cudaFree(ctx->d_ks));
+        ctx->d_ks = nullptr;
+        ctx->key_bytes -= rows * stride * sizeof(int32_t);
+    }
     return TFHE_GPU_OK;
 }
 
@@ -586,9 +601,9 @@ tfhe_gpu_status tfhe_gpu_tLweExtractLweSample(tfhe_gpu_ctx* ctx, int32_t* out,
 tfhe_gpu_status tfhe_gpu_lweKeySwitch(tfhe_gpu_ctx* ctx, int32_t* out, const int32_t* in,
                                       int32_t count, void* stream) {
     CHECK_CTX(ctx);
-    if (!ctx->d_ks) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     if (count < 0 || (count && (!out || !in))) return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
-    CK(ctx, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, in, out, count,
+    CK(ctx, launch_keyswitch(ctx->dp, ctx->ks_table(), in, out, count,
                              pick(ctx, stream)));
     return TFHE_GPU_OK;
 }
@@ -607,14 +622,14 @@ tfhe_gpu_status tfhe_gpu_tfhe_bootstrap_FFT(tfhe_gpu_ctx* ctx, int32_t* out, con
                                             void* stream) {
     CHECK_CTX(ctx);
     RET(need_bk(ctx, form));
-    if (!ctx->d_ks) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     if (count < 0 || (count && (!out || !x))) return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
     if (count == 0) return TFHE_GPU_OK;
     void* u;
     RET(ensure_scratch(ctx, 1, (size_t)count * (ctx->P.k * ctx->P.N + 1) * sizeof(int32_t), &u));
     cudaStream_t st = pick(ctx, stream);
     RET(run_bootstrap_woks(ctx, x, mu, (int32_t*)u, count, form, st));
-    CK(ctx, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, (const int32_t*)u, out, count,
+    CK(ctx, launch_keyswitch(ctx->dp, ctx->ks_table(), (const int32_t*)u, out, count,
                              st));
     return TFHE_GPU_OK;
 }
@@ -624,7 +639,7 @@ tfhe_gpu_status tfhe_gpu_bootstrap_tv(tfhe_gpu_ctx* ctx, int32_t* out, const int
                                       tfhe_gpu_form form, int32_t keyswitch, void* stream) {
     CHECK_CTX(ctx);
     RET(need_bk(ctx, form));
-    if (keyswitch && !ctx->d_ks) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    if (keyswitch && !ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     if (count < 0 || (count && (!out || !x || !tv)) || (tv_stride != 0 && tv_stride != ctx->P.N))
         return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
     if (count == 0) return TFHE_GPU_OK;
@@ -646,7 +661,7 @@ tfhe_gpu_status tfhe_gpu_bootstrap_tv(tfhe_gpu_ctx* ctx, int32_t* out, const int
     CK(ctx, launch_external_product(ctx->dp, (Form)form, kEpBlindRotate, ctx->tables, a,
                                     ctx->groups_per_cta[form], st));
     if (keyswitch)
-        CK(ctx, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, u, out, count, st));
+        CK(ctx, launch_keyswitch(ctx->dp, ctx->ks_table(), u, out, count, st));
     return TFHE_GPU_OK;
 }
 
@@ -673,7 +688,7 @@ tfhe_gpu_status tfhe_gpu_bootsMUX(tfhe_gpu_ctx* ctx, int32_t* out, const int32_t
                                   tfhe_gpu_form form, void* stream) {
     CHECK_CTX(ctx);
     RET(need_bk(ctx, form));
-    if (!ctx->d_ks) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     if (count < 0 || (count && (!out || !a || !b || !c))) return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
     if (count == 0) return TFHE_GPU_OK;
     const int n = ctx->P.n, nk = ctx->P.k * ctx->P.N;
@@ -693,7 +708,7 @@ tfhe_gpu_status tfhe_gpu_bootsMUX(tfhe_gpu_ctx* ctx, int32_t* out, const int32_t
     const int32_t* u1 = (const int32_t*)u;
     const int32_t* u2 = u1 + (size_t)count * (nk + 1);
     CK(ctx, launch_lwe_add2_const(u1, u2, (int32_t*)s, nk + 1, mu, count, st));
-    CK(ctx, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, (const int32_t*)s, out, count,
+    CK(ctx, launch_keyswitch(ctx->dp, ctx->ks_table(), (const int32_t*)s, out, count,
                              st));
     return TFHE_GPU_OK;
 }
@@ -754,7 +769,7 @@ tfhe_gpu_status tfhe_gpu_graph_gates_create(tfhe_gpu_ctx* ctx, const int32_t* ga
         return fail(ctx, TFHE_GPU_BAD_PARAM, "graph args");
     *result = nullptr;
     RET(need_bk(ctx, form));
-    if (!ctx->d_ks) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     const int n = ctx->P.n, nk = ctx->P.k * ctx->P.N;
     tfhe_gpu_graph* g = new tfhe_gpu_graph();
     g->ctx = ctx;

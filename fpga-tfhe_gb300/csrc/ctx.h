@@ -25,8 +25,13 @@ struct tfhe_gpu_ctx {
     void* d_tables = nullptr;  // transform tables: FP64 copy then FP32 copy
     Tables tables{};
     void* d_bk[kNumForms] = {nullptr, nullptr};
+    // key-switching table: its words in FP16 pieces for the tensor-core key
+    // switch (t = 8), or the rows
+    void* d_ks_tiles = nullptr;
     int32_t* d_ks = nullptr;
+    bool has_ks() const { return d_ks || d_ks_tiles; }
     int32_t ks_row_stride = 0;
+    tfhe_gb300::KsTable ks_table() const { return {d_ks, ks_row_stride, d_ks_tiles, d_err}; }
     // scratch slots, grown on demand
     void* d_scratch[4] = {nullptr, nullptr, nullptr, nullptr};
     size_t scratch_bytes[4] = {0, 0, 0, 0};

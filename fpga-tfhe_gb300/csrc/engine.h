@@ -120,11 +120,26 @@ cudaError_t launch_lagrange_addmul(const double* a, const double* b,
 // single launch or another shape is set.
 int blind_rotate_tail_start(Form f, int groups, int count);
 
-// Key switching: in (count x (kN+1)) -> out (count x (n+1)); ks rows are
-// `row_stride` int32 apart, layout [kN][t][base][row_stride].
-cudaError_t launch_keyswitch(const DevParams& P, const int32_t* ks,
-                             int32_t row_stride, const int32_t* in,
+// Key-switching table on the device: for t = 8 its words in FP16 pieces in
+// the tensor cores' order (tiles), for other t rows `row_stride` int32 apart,
+// layout [kN][t][base][row_stride]; the other pointer is null.  err: device
+// status word.
+struct KsTable {
+    const int32_t* rows;
+    int32_t row_stride;
+    const void* tiles;
+    int32_t* err;
+};
+// Key switching: in (count x (kN+1)) -> out (count x (n+1)).
+cudaError_t launch_keyswitch(const DevParams& P, const KsTable& ks, const int32_t* in,
                              int32_t* out, int count, cudaStream_t st);
+// Bytes of the pieces (0 when the parameters do not use them), their making
+// from the rows, and the tensor-core key switch (launch_keyswitch picks it).
+size_t keyswitch_tile_bytes(const DevParams& P);
+cudaError_t launch_keyswitch_tiles(const DevParams& P, const int32_t* ks, int32_t row_stride,
+                                   void* tiles, cudaStream_t st);
+cudaError_t launch_keyswitch_mma(const DevParams& P, const void* tiles, const int32_t* in, int32_t* out,
+                                 int count, int32_t* err, cudaStream_t st);
 
 // Finish n TGSW encryptions whose rows hold masks a and noise b = e (host
 // RNG, exact order): b += sum_i a_i * s_i (negacyclic, TLWE key s, N k

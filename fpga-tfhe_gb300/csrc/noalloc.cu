@@ -129,7 +129,7 @@ extern "C" tfhe_gpu_status tfhe_gpu_bootsGates_noalloc(tfhe_gpu_ctx* ctx, const 
         return set_error(ctx, TFHE_GPU_BAD_PARAM, "bootsGates_noalloc: bad arguments");
     if (!ctx->d_bk[form])
         return set_error(ctx, TFHE_GPU_NO_KEY, "bootstrapping key of this form not uploaded");
-    if (!ctx->d_ks) return set_error(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    if (!ctx->has_ks()) return set_error(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     const size_t w_in = (size_t)ctx->P.n + 1;
     const size_t w_ext = (size_t)ctx->P.k * ctx->P.N + 1;
     const size_t need = (size_t)count * (w_in + w_ext);
@@ -162,7 +162,7 @@ extern "C" tfhe_gpu_status tfhe_gpu_bootsGates_noalloc(tfhe_gpu_ctx* ctx, const 
     e = launch_external_product(ctx->dp, (Form)form, kEpBlindRotate, ctx->tables, a,
                                 ctx->groups_per_cta[form], st);
     if (e != cudaSuccess) return cuda_error(ctx, e, "blind rotation");
-    e = launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, u, out, count, st);
+    e = launch_keyswitch(ctx->dp, ctx->ks_table(), u, out, count, st);
     if (e != cudaSuccess) return cuda_error(ctx, e, "key switch");
     return TFHE_GPU_OK;
 }

@@ -492,17 +492,17 @@ tfhe_gpu_status enqueue(tfhe_gpu_server* s, Tick& T) {
         if (split && k1 > 0) {
             SCK(s, cudaEventRecord(ctx->ev_fork, st));
             SCK(s, cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-            SCK(s, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, s->d_u, s->d_out, k1, ctx->side));
+            SCK(s, launch_keyswitch(ctx->dp, ctx->ks_table(), s->d_u, s->d_out, k1, ctx->side));
             SCK(s, cudaEventRecord(ctx->ev_join, ctx->side));
         }
         if (split) SCK(s, rotate(split, nb - split));
         const int k0 = split && k1 > 0 ? k1 : 0;
-        SCK(s, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, s->d_u + (size_t)k0 * EW,
+        SCK(s, launch_keyswitch(ctx->dp, ctx->ks_table(), s->d_u + (size_t)k0 * EW,
                                 s->d_out + (size_t)k0 * W, nr - k0, st));
         if (nm) {
             SCK(s, launch_lwe_add2_const(s->d_u + (size_t)nr * EW, s->d_u + (size_t)(nr + nm) * EW,
                                          s->d_s, EW, 1 << 29, nm, st));
-            SCK(s, launch_keyswitch(ctx->dp, ctx->d_ks, ctx->ks_row_stride, s->d_s,
+            SCK(s, launch_keyswitch(ctx->dp, ctx->ks_table(), s->d_s,
                                     s->d_out + (size_t)nr * W, nm, st));
         }
         if (split && k1 > 0) SCK(s, cudaStreamWaitEvent(st, ctx->ev_join, 0));
