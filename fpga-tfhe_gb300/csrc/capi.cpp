@@ -408,7 +408,7 @@ tfhe_gpu_status tfhe_gpu_upload_keyswitch_key(tfhe_gpu_ctx* ctx, const int32_t* 
     const int n = ctx->P.n;
     const int stride = (n + 1 + 3) & ~3;
     const size_t rows = (size_t)ctx->P.k * ctx->P.N * ctx->P.ks_t * (1 << ctx->P.ks_basebit);
-    if (!ctx->has_ks()) {
+    if (!ctx->d_ks) {
         CK(ctx, cudaMalloc(&ctx->d_ks, rows * stride * sizeof(int32_t)));
         ctx->key_bytes += rows * stride * sizeof(int32_t);
     }
