@@ -96,6 +96,12 @@ __device__ __forceinline__ void st_async_f2(uint32_t raddr, float x, float y, ui
                  : "memory");
 }
 
+__device__ __forceinline__ void st_async_i2(uint32_t raddr, int32_t x, int32_t y, uint32_t rbar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(raddr),
+                 "r"(x), "r"(y), "r"(rbar)
+                 : "memory");
+}
+
 // The same for 16 bytes (two doubles, as four 32-bit words).
 __device__ __forceinline__ void st_async_d2(uint32_t raddr, double x, double y, uint32_t rbar) {
     asm volatile(

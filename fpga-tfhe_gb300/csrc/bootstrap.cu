@@ -1614,6 +1614,284 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
 }
 
 // ----------------------------------------------------------------------
+// The FP64 form's blind rotation over a cluster of eight CTAs (lowest FP64
+// latency).  One SM's FP64 unit takes 19 clocks per warp instruction (64 for
+// a warp alone), so a step's latency is the FP64 work per SM; here a step's
+// 5,000 warp instructions are spread over eight SMs in warps of four per SM.
+//
+//   CTA p < 2l transforms row p's digits (polynomial p / l, level p % l): 128
+//   threads, each computing four of a butterfly's eight outputs (its parity,
+//   the same for a whole warp: dft8_parity), the inputs exchanged through
+//   shared memory, so no operation is done twice.  Positions 64b .. 64b + 63
+//   of the result go to CTA b.
+//   CTA b multiplies all 2l rows, in row order, at its 64 positions for both
+//   output polynomials, one (position, output) a thread, and runs the inverse
+//   passes C' and B', which stay within those positions, one output of a
+//   butterfly a thread (dft8_one, the output pair the same for a warp).
+//   Point t of the block's results goes to CTA t / 8.
+//   CTA m runs pass A' for points t = 8m .. 8m + 7, truncates, adds into the
+//   coefficients it keeps in registers (t + 64q and + 512), and sends them to
+//   the l CTAs that decompose that polynomial.
+//
+// The three exchanges of a step are asynchronous stores (st.async) counted
+// in bytes on the receiver's mbarrier, each into a single buffer: data of
+// step k + 1 can only come after every CTA has received all of step k's
+// coefficients, and each of those was sent after its sender had read its
+// step-k digits and points.  All waits are bounded.
+// Every product, sum and rounding is the other FP64 shapes', on the same
+// operands, so the ciphertexts agree bit for bit.
+// Measured: one ciphertext 20.3 -> 6.2 ms against the two-SM cluster kernel.
+// ----------------------------------------------------------------------
+template <int L>
+struct Cluster8F64Plan {
+    static constexpr int kThreads = 128;
+    static constexpr size_t acc_off = kHotSize * sizeof(cpx<double>);      // polynomial p / l: (x, x + 512) pairs
+    static constexpr size_t x_off = acc_off + kN * sizeof(int32_t);        // transform buffers, ping and pong
+    static constexpr size_t d_off = x_off + 2 * kScratchStride * sizeof(cpx<double>);  // [row][q][8] digits received
+    static constexpr size_t o_off = d_off + 2 * L * 64 * sizeof(cpx<double>);  // [output][64] block buffers, two
+    static constexpr size_t p_off = o_off + 2 * 2 * 72 * sizeof(cpx<double>);  // [output][block][8] points received
+    static constexpr size_t bar_off = p_off + 2 * 64 * sizeof(cpx<double>);    // 3 mbarriers, abort flag
+    static constexpr size_t total = bar_off + 3 * sizeof(uint64_t) + 16;
+    static_assert(acc_off % 16 == 0 && d_off % 16 == 0 && p_off % 16 == 0, "16-byte stores");
+};
+
+// one output of the 8-point butterfly v for a thread of class C = its warp
+template <int S>
+__device__ __forceinline__ cpx<double> dft8_by_warp(const cpx<double> (&v)[8], int cls, bool minus) {
+    switch (cls) {
+    case 0: return dft8_one<S, 0>(v, minus);
+    case 1: return dft8_one<S, 1>(v, minus);
+    case 2: return dft8_one<S, 2>(v, minus);
+    default: return dft8_one<S, 3>(v, minus);
+    }
+}
+
+// Barrier of the 128 threads; the two parities reach it from different code.
+__device__ __forceinline__ void parity_sync() { asm volatile("barrier.sync 1, 128;" ::: "memory"); }
+
+// Forward transform of one polynomial's digits by 128 threads: (t, H) with
+// H the parity of the outputs the thread computes.  In: w[k] = digit of point
+// t + 64 (4H + k).  Out: y[k] = position 8t + 2k + H.
+template <int H>
+__device__ __forceinline__ void forward_parity(cpx<double> (&w)[4], cpx<double> (&y)[4], cpx<double>* x0,
+                                               cpx<double>* x1, const FftTwiddles<double>& tw, int t) {
+    cpx<double> v[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (4 * H + k) w[k] = cmul_const(w[k], twist_c<double>(4 * H + k));
+        x0[spad(t + 64 * (4 * H + k))] = w[k];
+    }
+    parity_sync();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = x0[spad(t + 64 * q)];
+    dft8_parity<1, H>(v, y);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x1[spad(t + 64 * (2 * k + H))] = cmul_table(y[k], tw.a[(2 * k + H) * 64 + t]);
+    parity_sync();
+    const int b = t >> 3, j = t & 7;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = x1[spad(64 * b + j + 8 * q)];
+    dft8_parity<1, H>(v, y);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (2 * k + H) y[k] = cmul_table(y[k], tw.b[(2 * k + H) * 8 + j]);
+        x0[spad(64 * b + j + 8 * (2 * k + H))] = y[k];
+    }
+    parity_sync();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = x0[spad(8 * t + q)];
+    dft8_parity<1, H>(v, y);
+}
+
+template <int L>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::kThreads, 1)
+    k_blind_rotate_cluster8_f64(KParams kp, Tables T, EpArgs a) {
+    namespace cg = cooperative_groups;
+    using Plan = Cluster8F64Plan<L>;
+    constexpr int kRows = 2 * L;
+    extern __shared__ __align__(128) char smem[];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int m = (int)cluster.block_rank();
+    cpx<double>* tables = reinterpret_cast<cpx<double>*>(smem);
+    int2* acc = reinterpret_cast<int2*>(smem + Plan::acc_off);
+    cpx<double>* x0 = reinterpret_cast<cpx<double>*>(smem + Plan::x_off);
+    cpx<double>* x1 = x0 + kScratchStride;
+    cpx<double>* din = reinterpret_cast<cpx<double>*>(smem + Plan::d_off);
+    cpx<double>* o0 = reinterpret_cast<cpx<double>*>(smem + Plan::o_off);
+    cpx<double>* o1 = o0 + 2 * 72;
+    cpx<double>* pin = reinterpret_cast<cpx<double>*>(smem + Plan::p_off);
+    uint64_t* bar_acc = reinterpret_cast<uint64_t*>(smem + Plan::bar_off);  // coefficients received
+    uint64_t* bar_d = bar_acc + 1;                                          // digits received
+    uint64_t* bar_p = bar_acc + 2;                                          // points received
+    volatile int* abort = reinterpret_cast<volatile int*>(bar_acc + 3);
+    const int c = blockIdx.x >> 3;
+    const int u = threadIdx.x, warp = u >> 5, lane = u & 31;
+    const int n = kp.n;
+    const bool forward = m < kRows;
+    const int jp = m / L, lev = m - jp * L;  // forward: polynomial and level
+    load_hot_tables<double>(tables, T);
+
+    // coefficient pairs kept by this thread: output wj, point 8m + wt, q = wq
+    // (x = 8m + wt + 64 wq and x + 512); the same thread numbering serves the
+    // inverse passes: output wj, butterfly wt, butterfly output wq
+    const int wj = (lane >> 3) & 1, wt = lane & 7;
+    const bool minus = lane >= 16;
+    const int wq = 2 * (warp & 1) + (warp >> 1) + (minus ? 4 : 0);
+    uint32_t own0, own1;
+    {
+        const int x = 8 * m + wt + 64 * wq;
+        const int32_t* src = a.acc_in ? a.acc_in + (size_t)c * 2 * kN : nullptr;
+        const int barb = src ? 0 : mod_switch_2n(a.x[(size_t)c * (n + 1) + n]);
+        const auto start = [&](int j, int i) -> int32_t {
+            return src ? src[j * kN + i] : j == 0 ? 0 : test_vector_coef(a, c, barb, i);
+        };
+        own0 = (uint32_t)start(wj, x);
+        own1 = (uint32_t)start(wj, x + kHalf);
+        if (forward)
+            for (int i = u; i < kHalf; i += Plan::kThreads) acc[i] = make_int2(start(jp, i), start(jp, i + kHalf));
+    }
+    if (u == 0) {
+        mbar_init(bar_acc, 1);
+        mbar_init(bar_d, 1);
+        mbar_init(bar_p, 1);
+        *abort = 0;
+        fence_mbar_init();
+    }
+    cluster.sync();  // every CTA's barriers initialised before any store
+
+    const FftTwiddles<double> tw = hot_twiddles<double>(tables);
+    const int halfBg = 1 << (kp.Bgbit - 1);
+    const uint32_t mask = (1u << kp.Bgbit) - 1;
+    const int decal = 32 - (lev + 1) * kp.Bgbit;
+    const cpx<double>* gsw = reinterpret_cast<const cpx<double>*>(a.gsw);
+    const size_t step_elems = (size_t)kRows * 2 * kHalf;
+    const int32_t* bara = a.bara ? a.bara + (size_t)c * n : nullptr;
+    const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
+    const int32_t* rot = bara ? bara : xs;
+    const auto wait_for = [&](uint64_t* bar, uint32_t parity) {
+        if (!mbar_wait_cluster_bounded(bar, parity, abort)) {
+            *abort = 1;
+            atomicExch(a.err, 3);
+        }
+        __syncwarp();
+    };
+    int32_t rot_next = rot[0];
+    uint32_t k = 0;  // steps taken (the same in all CTAs)
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+        const int ai = bara ? rot_next : mod_switch_2n(rot_next);
+        if (i + 1 < n) rot_next = rot[i + 1];
+        if (ai == 0) continue;  // tfhe_blindRotate_FFT.cpp:114 (uniform over the cluster)
+        if (u == 0) {
+            mbar_arrive_expect_tx(bar_d, kRows * 64 * sizeof(cpx<double>));
+            mbar_arrive_expect_tx(bar_p, 2 * 64 * sizeof(cpx<double>));
+        }
+        // this step's key values at (output mj, position 64m + 8 mt + mq)
+        const int mj = u >> 6, mq = (u >> 3) & 7, mt = u & 7;
+        double2 kk[kRows];
+        {
+            const double2* g2 = reinterpret_cast<const double2*>(gsw + (size_t)i * step_elems + mj * kHalf) +
+                                key_index<double>(8 * m + mt, mq);
+#pragma unroll
+            for (int p = 0; p < kRows; ++p) kk[p] = __ldg(g2 + (size_t)p * 2 * kHalf);
+        }
+        if (forward) {
+            if (k > 0) wait_for(bar_acc, (k - 1) & 1);
+            if (u == 0) mbar_arrive_expect_tx(bar_acc, kN * sizeof(int32_t));
+            __syncwarp();
+            const int t = u & 63, hp = u >> 6;
+            cpx<double> w[4], y[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int s = t + 64 * (4 * hp + q);
+                const int2 p = acc[s];
+                const int rs = s - ai;
+                const int2 v = acc[rs & (kHalf - 1)];
+                const uint32_t v0 = (uint32_t)(rs & kHalf ? v.y : v.x), v1 = (uint32_t)(rs & kHalf ? v.x : v.y);
+                const uint32_t u0 = (rs & kN ? 0u - v0 : v0) - (uint32_t)p.x + kp.offset;
+                const uint32_t u1 = ((rs + kHalf) & kN ? 0u - v1 : v1) - (uint32_t)p.y + kp.offset;
+                w[q] = digit_pair<double>(u0, u1, decal, mask, halfBg);
+            }
+            if (hp == 0) forward_parity<0>(w, y, x0, x1, tw, t);
+            else forward_parity<1>(w, y, x0, x1, tw, t);
+            const uint32_t dst = cluster_map(smem_u32(din), (uint32_t)(t >> 3));
+            const uint32_t dbar = cluster_map(smem_u32(bar_d), (uint32_t)(t >> 3));
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                st_async_d2(dst + (uint32_t)((m * 64 + (2 * q + hp) * 8 + (t & 7)) * sizeof(cpx<double>)), y[q].x,
+                            y[q].y, dbar);
+        }
+        wait_for(bar_d, k & 1);
+        {
+            cpx<double> o = {0.0, 0.0};
+#pragma unroll
+            for (int p = 0; p < kRows; ++p) {
+                const cpx<double> z = cmul_table(din[p * 64 + mq * 8 + mt], cpx<double>{kk[p].x, kk[p].y});
+                o = {__dadd_rn(o.x, z.x), __dadd_rn(o.y, z.y)};
+            }
+            o0[mj * 72 + 9 * mt + mq] = o;
+        }
+        __syncthreads();
+        cpx<double> v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = o0[wj * 72 + 9 * wt + q];
+        // pass C' of butterfly wt, output wq, times pass B''s twiddle
+        o1[wj * 72 + 9 * wt + wq] = cmulc_any(dft8_by_warp<-1>(v, warp, minus), tw.b[wt * 8 + wq]);
+        __syncthreads();
+        // pass B' of butterfly j = wt (positions j + 8r), output wq, times pass A''s twiddle
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = o1[wj * 72 + 9 * q + wt];
+        {
+            const cpx<double> z = cmulc_any(dft8_by_warp<-1>(v, warp, minus), tw.a[m * 64 + wt + 8 * wq]);
+            st_async_d2(cluster_map(smem_u32(pin), (uint32_t)wq) +
+                            (uint32_t)(((wj * 8 + m) * 8 + wt) * sizeof(cpx<double>)),
+                        z.x, z.y, cluster_map(smem_u32(bar_p), (uint32_t)wq));
+        }
+        // pass A' of point 8m + wt, output wq
+        wait_for(bar_p, k & 1);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = pin[(wj * 8 + q) * 8 + wt];
+        {
+            cpx<double> z = dft8_by_warp<-1>(v, warp, minus);
+            cpx<double> un = {1.0, 0.0};
+#pragma unroll
+            for (int q = 1; q < 8; ++q)
+                if (wq == q) un = twist_c<double>(q);
+            z = cmulc_any(z, un);
+            own0 += trunc_div512(z.x);
+            own1 += trunc_div512(z.y);
+            const int x = 8 * m + wt + 64 * wq;
+#pragma unroll
+            for (int lv = 0; lv < L; ++lv) {
+                const uint32_t rank = (uint32_t)(wj * L + lv);
+                st_async_i2(cluster_map(smem_u32(acc), rank) + (uint32_t)(x * sizeof(int2)), (int32_t)own0,
+                            (int32_t)own1, cluster_map(smem_u32(bar_acc), rank));
+            }
+        }
+        ++k;
+    }
+    const int x = 8 * m + wt + 64 * wq;
+    if (a.acc_out) {
+        int32_t* dst = a.acc_out + (size_t)c * 2 * kN + wj * kN;
+        dst[x] = (int32_t)own0;
+        dst[x + kHalf] = (int32_t)own1;
+    }
+    if (a.lwe_out) {
+        // tLweExtractLweSample: a'_0 = a_0, a'_j = -a_{N-j}, b' = b_0
+        int32_t* dst = a.lwe_out + (size_t)c * (kN + 1);
+        if (wj == 0) {
+            if (x == 0) dst[0] = (int32_t)own0;
+            else dst[kN - x] = (int32_t)(0u - own0);
+            dst[kHalf - x] = (int32_t)(0u - own1);
+        } else if (x == 0) {
+            dst[kN] = (int32_t)own0;
+        }
+    }
+    if (forward && k > 0) wait_for(bar_acc, (k - 1) & 1);  // the last coefficients landed
+    cluster.sync();  // no CTA leaves while another could still address its shared memory
+}
+
+// ----------------------------------------------------------------------
 // The FP64 form's blind rotation, one ciphertext per CTA: 2l groups of 64
 // threads run a step's 2l forward transforms at once, then groups 0 and 1
 // multiply all 2l rows in row order with their output polynomial's part of
@@ -2358,6 +2636,19 @@ cudaError_t launch_spread2_f64(const DevParams& P, const Tables& T, const EpArgs
     return cudaGetLastError();
 }
 
+// FP64: one ciphertext per cluster of eight CTAs
+template <int L>
+cudaError_t launch_cluster8_f64(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
+    if (a.count <= 0) return cudaSuccess;
+    const KParams kp = make_kparams(P);
+    using Plan = Cluster8F64Plan<L>;
+    auto kern = k_blind_rotate_cluster8_f64<L>;
+    cudaError_t e = set_smem(kern, Plan::total);
+    if (e != cudaSuccess) return e;
+    kern<<<8 * a.count, Plan::kThreads, Plan::total, st>>>(kp, T, a);
+    return cudaGetLastError();
+}
+
 // FP64: one ciphertext per CTA
 template <int L>
 cudaError_t launch_spread_f64(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
@@ -2431,12 +2722,13 @@ cudaError_t launch_auto_fp32(const DevParams& P, const Tables& T, const EpArgs& 
 
 // Automatic shape of an FP64 blind rotation.  Every shape gives the same
 // ciphertexts, so only time decides.  Measured per launch (default set): the
-// cluster kernel 20.4 ms for up to one ciphertext per two SMs; the
-// one-per-CTA kernel 29.8 ms a wave of one per SM; the 3-per-CTA kernel with
+// eight-SM cluster kernel 6.2 ms for up to 15 ciphertexts, 10.6 ms to 32, 15.6
+// ms to 48, 20.9 ms at 57; the two-SM cluster kernel 20.3 ms for up to one
+// ciphertext per two SMs; the one-per-CTA kernel 29.8 ms a wave of one per SM; the 3-per-CTA kernel with
 // L2-direct key reads 87.0 ms a wave of three per SM (3 waves of the former
 // take 89.3 ms).  So whole waves of three per SM, and a remainder of up to
 // two per SM on the one-per-CTA kernel, of up to one per two SMs on the
-// cluster kernel.
+// two-SM cluster kernel, of up to 48 on the eight-SM one.
 template <int L>
 cudaError_t launch_auto_fp64(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
     const int wave = 3 * kSmCount;
@@ -2449,6 +2741,7 @@ cudaError_t launch_auto_fp64(const DevParams& P, const Tables& T, const EpArgs& 
     }
     const EpArgs tail = slice_blind_rotate(P, a, full, a.count - full);
     if (tail.count > kSmCount / 2) return launch_spread_f64<L>(P, T, tail, st);
+    if (tail.count <= 48) return launch_cluster8_f64<L>(P, T, tail, st);
     return launch_spread2_f64<L>(P, T, tail, st);
 }
 

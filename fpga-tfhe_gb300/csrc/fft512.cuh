@@ -187,6 +187,79 @@ __device__ __forceinline__ void dft8(cpx<R> (&v)[8]) {
     }
 }
 
+// FP64 complex products with their fused operations spelt out.  Which product
+// of a sum of two is fused is otherwise the compiler's choice, which differs
+// between kernels; these are the choices it makes in the whole-transform FP64
+// kernels (fft512_forward_ip1 and so on), found by emulating their outputs:
+// a w for a table value w, a c for a constant c, a conj(w).
+__device__ __forceinline__ cpx<double> cmul_table(cpx<double> a, cpx<double> w) {
+    return {__fma_rn(a.x, w.x, -__dmul_rn(a.y, w.y)), __fma_rn(a.x, w.y, __dmul_rn(a.y, w.x))};
+}
+__device__ __forceinline__ cpx<double> cmul_const(cpx<double> a, cpx<double> c) {
+    return {__fma_rn(a.x, c.x, -__dmul_rn(a.y, c.y)), __fma_rn(a.y, c.x, __dmul_rn(a.x, c.y))};
+}
+__device__ __forceinline__ cpx<double> cmulc_any(cpx<double> a, cpx<double> w) {
+    return {__fma_rn(a.x, w.x, __dmul_rn(a.y, w.y)), __fma_rn(a.y, w.x, -__dmul_rn(a.x, w.y))};
+}
+
+// Parts of dft8 for butterflies shared by several threads, with its
+// operations on the same operands (so the same bits): the outputs of one
+// parity (q = 2k + H into y[k]), and the two outputs q = 2(C & 1) + (C >> 1)
+// and q + 4, of which `minus` picks the second.
+template <int S, int H, typename R>
+__device__ __forceinline__ void dft8_quad(const cpx<R> (&v)[8], cpx<R> (&b)[4]) {
+    if constexpr (H == 0) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) b[r] = cadd(v[r], v[r + 4]);
+    } else {
+        const R h = (R)0.70710678118654752440084436210485;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) b[r] = csub(v[r], v[r + 4]);
+        {
+            const R x = b[1].x, y = b[1].y;
+            b[1] = {(x - S * y) * h, (y + S * x) * h};
+        }
+        {
+            const R x = b[2].x, y = b[2].y;
+            b[2] = {-S * y, S * x};
+        }
+        {
+            const R x = b[3].x, y = b[3].y;
+            b[3] = {(-x - S * y) * h, (S * x - y) * h};
+        }
+    }
+}
+template <int S, int H, typename R>
+__device__ __forceinline__ void dft8_parity(const cpx<R> (&v)[8], cpx<R> (&y)[4]) {
+    cpx<R> b[4];
+    dft8_quad<S, H>(v, b);
+    const cpx<R> e0 = cadd(b[0], b[2]), e1 = csub(b[0], b[2]), e2 = cadd(b[1], b[3]);
+    const cpx<R> d = csub(b[1], b[3]);
+    const cpx<R> e3 = {-S * d.y, S * d.x};
+    y[0] = cadd(e0, e2);
+    y[1] = cadd(e1, e3);
+    y[2] = csub(e0, e2);
+    y[3] = csub(e1, e3);
+}
+__device__ __forceinline__ double flip_sign(double x, bool minus) {
+    return __hiloint2double(__double2hiint(x) ^ (minus ? (int)0x80000000 : 0), __double2loint(x));
+}
+template <int S, int C>
+__device__ __forceinline__ cpx<double> dft8_one(const cpx<double> (&v)[8], bool minus) {
+    cpx<double> b[4];
+    dft8_quad<S, (C >> 1)>(v, b);
+    cpx<double> e, f;
+    if constexpr ((C & 1) == 0) {
+        e = cadd(b[0], b[2]);
+        f = cadd(b[1], b[3]);
+    } else {
+        e = csub(b[0], b[2]);
+        const cpx<double> d = csub(b[1], b[3]);
+        f = {-S * d.y, S * d.x};
+    }
+    return cadd(e, cpx<double>{flip_sign(f.x, minus), flip_sign(f.y, minus)});
+}
+
 __device__ __forceinline__ void group_sync(int bar_id) {
     asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(kFftThreads) : "memory");
 }

@@ -131,8 +131,9 @@ size_t tfhe_gpu_device_bytes(const tfhe_gpu_ctx* ctx);
  *       mbarrier (lowest latency: about 1.33 ms for a single gate's blind
  *       rotation).
  * FP64: 0 = automatic (the default): whole waves of three ciphertexts per SM
- * on 3; a remainder of up to one per two SMs on the two-SM cluster kernel, of
- * up to two per SM on a one-per-CTA kernel, else one more wave of 3; 3 =
+ * on 3; a remainder of up to 48 on an eight-SM cluster kernel, of up to one
+ * per two SMs on the two-SM cluster kernel, of up to two per SM on a
+ * one-per-CTA kernel, else one more wave of 3; 3 =
  * L2-direct key reads, 3 per CTA;
  * 4 = shared key ring fed in line; 16 = the cluster kernel (one owner group
  * per CTA: the FP64 key has one part).  Engine tuning knob, no counterpart

@@ -59,8 +59,8 @@ def _uniform(torch, seed, *shape):
     return torch.randint(-2 ** 31, 2 ** 31, shape, generator=g, device="cuda", dtype=torch.int32)
 
 
-# FP64: 76 | 77 .. 304 | 305 .. 456 | 457 is a whole wave and a remainder
-@pytest.mark.parametrize("params,count", [("default", 77), ("stress", 76), ("stress", 153), ("stress", 305),
+# FP64: 48 | 49 .. 76 | 77 .. 304 | 305 .. 456 | 457 is a whole wave and a remainder
+@pytest.mark.parametrize("params,count", [("default", 1), ("stress", 16), ("default", 48), ("stress", 49), ("default", 77), ("stress", 76), ("stress", 153), ("stress", 305),
                                           ("stress", 457), ("stress", 533)])
 def test_fp64_automatic_shape_matches_l2_direct(engines, torch_cuda, params, count):
     torch = torch_cuda
@@ -70,7 +70,7 @@ def test_fp64_automatic_shape_matches_l2_direct(engines, torch_cuda, params, cou
     assert (got == _bootstraps(torch, e, "fp64", 3, x)).all()
 
 
-@pytest.mark.parametrize("count", [80])
+@pytest.mark.parametrize("count", [5, 80])
 def test_fp64_blind_rotate_from_accumulators(engines, torch_cuda, count):
     torch = torch_cuda
     e = engines("stress")
