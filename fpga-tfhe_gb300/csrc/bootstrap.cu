@@ -1105,155 +1105,267 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
 }
 
 // ----------------------------------------------------------------------
-// Blind rotation with one ciphertext over 2l groups (lowest latency).
+// Blind rotation with one ciphertext per CTA (low latency, up to one per SM).
+// Split-FP32 only.
 //
-// Group g = (jp, lev) = (g / l, g % l) decomposes input polynomial jp at
-// level lev, runs that one forward transform and writes the transformed
-// digits D_g to shared memory.  After a CTA barrier, owner group (j, pt) =
-// (g / 2, g % 2) for g < 4 multiplies all 2l of them with part (j, pt) of
-// each key row, transforms back, rounds, and adds its part into the
-// accumulator with integer shared-memory atomics (exact mod 2^32 in any
-// order, so the result does not depend on timing).  The owners issue their
-// key loads (4 float4 per row, from L2) before the barrier, so the latency
-// overlaps the other groups' transforms; the next step's rows are
-// prefetched into L2.  A step's critical path is one forward transform, 2l
-// rows of products and one inverse transform, against the pair kernel's l
-// forward and PARTS inverse transforms.  Split-FP32 only.
+// l sets of 128 threads run transforms in lane pairs (fft512_forward_duo):
+// the two lanes of a pair hold the same point of two transforms and share
+// addresses of the accumulator and the digits.  Set j < 2 decomposes
+// polynomial j and transforms its levels 0 and 1, set 2 (l = 3) level 2 of
+// both polynomials; each writes its transformed digits D to shared memory.
+// After a barrier, sets 0 and 1 own the output polynomials: lane pair t
+// multiplies all 2l rows in row order, the high key part in the even lane and
+// the low part in the odd one, which read the same D, transforms both back
+// and rounds.  The lanes then exchange halves, so that the even one has the
+// whole sum of coefficients t + 64q and the odd one that of the 512 above,
+// kept in registers and written out for the next step's rotation.  A producer
+// warp copies each step's key rows into shared memory (one 4 KB part of a row
+// a lane) as soon as the owners have used the last step's.  The products are
+// summed in the same order as in every other shape, so the ciphertexts are
+// the same bit for bit.
+//
+// What bounds it: the shared-memory pipe (about 4,300 wavefronts of a step's
+// 5,200 clocks: the key values written and read 1,536, the transforms'
+// exchanges 1,280, the digits 580) and the chain of a step's phases.
+// Measured against the form with one transform per 64 threads, the high and
+// the low part in different groups, keys loaded into registers (the loads
+// held the load/store unit for 600 clocks a step) and accumulated by
+// shared-memory atomics: 1.755 -> 1.587 ms for 152 ciphertexts; the twiddles
+// in registers instead of shared memory are 0.054 ms of that.
 // ----------------------------------------------------------------------
 template <int L>
 struct SpreadPlan {
-    static constexpr int kGroups = 2 * L;
-    static constexpr size_t tables = kHotSize * sizeof(cpx<float>);
-    static constexpr size_t acc_off = tables;
-    static constexpr size_t d_off = acc_off + 2 * kN * sizeof(int32_t);
-    static constexpr size_t scratch_off = d_off + kGroups * kHalf * sizeof(cpx<float>);
-    static constexpr size_t scratch = 2 * kScratchStride * sizeof(cpx<float>);
-    static constexpr size_t total = scratch_off + kGroups * scratch;
+    static_assert(L == 2 || L == 3, "levels 0, 1 in lane pairs, level 2 apart");
+    static constexpr int kSets = L;
+    static constexpr int kThreads = kDuoThreads * kSets + 32;  // and the producer warp
+    // a step's key values, [row][polynomial][part], each part 64 bytes round
+    // so that the two lanes of a pair fall on different banks
+    static constexpr int kKeyPart = kHalf * sizeof(cpx<float>) + 64;
+    static constexpr int kKeyParts = 2 * L * 2 * 2;
+    static constexpr int kDA = 2 * kHalf;               // digits of levels 0, 1 of a polynomial: [q][t][level]
+    static constexpr int kDB = L == 3 ? kHalf + 8 : 0;  // of level 2: [q][t], the next polynomial's 64 bytes round
+    static constexpr int kD = kDA + kDB;
+    static constexpr size_t acc_off = kHotSize * sizeof(cpx<float>);
+    static constexpr size_t d_off = acc_off + 2 * 2 * kN * sizeof(int32_t);  // two quadrants, see spread_put
+    static constexpr size_t x_off = d_off + 2 * kD * sizeof(cpx<float>);
+    static constexpr size_t key_off = x_off + kSets * kDuoSlots * sizeof(cpx<float>);
+    static constexpr size_t bar_off = key_off + (size_t)kKeyParts * kKeyPart;  // 2 mbarriers, abort flag
+    static constexpr size_t total = bar_off + 2 * sizeof(uint64_t) + 16;
+    static_assert(d_off % 16 == 0 && kD * sizeof(cpx<float>) % 16 == 0, "16-byte digit loads");
+    static_assert(key_off % 16 == 0 && kKeyParts <= 32, "bulk copies, one a lane");
 };
 
+// The accumulator in shared memory: for every s in [0, N) the pair (c(s),
+// c(s + N/2)) of both polynomials, c the coefficients continued by X^N = -1,
+// so that a rotation reads a folded point with one 64-bit load and needs only
+// a sign.  With A and B the coefficients u and u + 512 (u < 512), s = u holds
+// (A, B) and s = u + 512 holds (B, -A).
+__device__ __forceinline__ int spread_word(int j, int x) {  // of coefficient x < N
+    return ((x & (kHalf - 1)) * 2 + j) * 2 + (x >> 9);
+}
+__device__ __forceinline__ void spread_put(int32_t* acc, int j, int x, uint32_t v) {
+    const int half = x >> 9;
+    int32_t* w = acc + ((x & (kHalf - 1)) * 2 + j) * 2;
+    w[half] = (int32_t)v;
+    w[kHalf * 4 + 1 - half] = (int32_t)(half ? v : 0u - v);
+}
+// X^a - 1 applied to the folded point t + 64r of polynomial j, plus the
+// gadget offset: r0 for coefficient t + 64r, r1 for that + 512.
+__device__ __forceinline__ void rotated_pair(const int32_t* acc, int j, int t, int r, int a, uint32_t offset,
+                                             uint32_t& r0, uint32_t& r1) {
+    const int2* src = reinterpret_cast<const int2*>(acc) + j;
+    const int s = t + 64 * r - a;
+    const int2 w = src[(s & (kN - 1)) * 2];
+    const int2 p = src[(t + 64 * r) * 2];
+    const uint32_t m = (uint32_t)((s << 21) >> 31);  // all ones when s mod 2N >= N
+    r0 = ((uint32_t)w.x ^ m) - (uint32_t)p.x + (offset - m);
+    r1 = ((uint32_t)w.y ^ m) - (uint32_t)p.y + (offset - m);
+}
+
 template <int L>
-__global__ void __launch_bounds__(128 * L, 1) k_blind_rotate_spread(KParams kp, Tables T, EpArgs a) {
+__global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spread(KParams kp, Tables T, EpArgs a) {
     using Plan = SpreadPlan<L>;
     constexpr int kRows = 2 * L;
     constexpr int kRowElems = 2 * 2 * kHalf;  // complex values per key row
     extern __shared__ __align__(128) char smem[];
     cpx<float>* tables = reinterpret_cast<cpx<float>*>(smem);
     int32_t* acc = reinterpret_cast<int32_t*>(smem + Plan::acc_off);
-    cpx<float>* dsh = reinterpret_cast<cpx<float>*>(smem + Plan::d_off);  // [g][q][t]
+    cpx<float>* dsh = reinterpret_cast<cpx<float>*>(smem + Plan::d_off);
+    uint64_t* kfull = reinterpret_cast<uint64_t*>(smem + Plan::bar_off);  // the step's key values landed
+    uint64_t* kfree = kfull + 1;                                          // every owner warp has used them
+    volatile int* abort = reinterpret_cast<volatile int*>(kfull + 2);
     const int c = blockIdx.x;
-    const int g = threadIdx.x >> 6, t = threadIdx.x & 63;
-    const int jp = g / L, lev = g - jp * L;
-    const bool owner = g < 4;
-    const int oj = g >> 1, opt = g & 1;
+    const int set = threadIdx.x >> 7, e = threadIdx.x & 1, t = (threadIdx.x & 127) >> 1;
+    const bool owner = set < 2;          // also the sets with levels 0 and 1 of one polynomial
+    const int jp = owner ? set : e;      // polynomial this lane decomposes
+    const int lev = owner ? e : 2;       // at this level; owners: output polynomial `set`, key part e
     const int n = kp.n;
     load_hot_tables<float>(tables, T);
     if (a.acc_in) {
         const int32_t* src = a.acc_in + (size_t)c * 2 * kN;
-        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x) acc[i] = src[i];
+        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x)
+            spread_put(acc, i >> 10, i & (kN - 1), (uint32_t)src[i]);
     } else {
         const int32_t* xs = a.x + (size_t)c * (n + 1);
         const int barb = mod_switch_2n(xs[n]);
         for (int i = threadIdx.x; i < kN; i += blockDim.x) {
-            acc[i] = 0;
-            acc[kN + i] = test_vector_coef(a, c, barb, i);
+            spread_put(acc, 0, i, 0u);
+            spread_put(acc, 1, i, (uint32_t)test_vector_coef(a, c, barb, i));
         }
+    }
+    if (threadIdx.x == 0) {
+        mbar_init(kfull, 1);
+        mbar_init(kfree, 8);  // owner warps
+        *abort = 0;
+        fence_mbar_init();
     }
     __syncthreads();
 
-    const FftTwiddles<float> tw = hot_twiddles<float>(tables);
-    const FftIdx ix = make_fft_idx(t);
-    const FftScratch<float> sc = scratch_at<float>(smem + Plan::scratch_off + (size_t)g * Plan::scratch);
-    const int bar_id = 1 + g;
-    const int halfBg = 1 << (kp.Bgbit - 1);
-    const uint32_t mask = (1u << kp.Bgbit) - 1;
-    const int decal = 32 - (lev + 1) * kp.Bgbit;
     const cpx<float>* gsw = reinterpret_cast<const cpx<float>*>(a.gsw);
     const size_t step_elems = (size_t)kRows * kRowElems;
-    const int32_t* bara = a.bara ? a.bara + (size_t)c * n : nullptr;
-    const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
-    const int32_t* rot = bara ? bara : xs;
-    int32_t rot_next = rot[0];
-    if (threadIdx.x < kRows) bulk_prefetch_l2(gsw + (size_t)threadIdx.x * kRowElems, kRowElems * sizeof(cpx<float>));
+    const auto gave_up = [&]() {
+        *abort = 1;
+        atomicExch(a.err, 3);
+    };
+    if (set == Plan::kSets) {
+        const int u = threadIdx.x & 31;
+        const cpx<float>* src = gsw + (size_t)u * kHalf;  // parts lie in order, row by row
+        int i = 0;
 #pragma unroll 1
-    for (int i = 0; i < n; ++i) {
-        const int ai = bara ? rot_next : mod_switch_2n(rot_next);
-        if (i + 1 < n) rot_next = rot[i + 1];
-        if (ai == 0) continue;  // tfhe_blindRotate_FFT.cpp:114 (uniform over the CTA)
-        const cpx<float>* step_keys = gsw + (size_t)i * step_elems;
-        if (i + 1 < n && threadIdx.x < kRows)  // the next step's rows into L2
-            bulk_prefetch_l2(step_keys + step_elems + (size_t)threadIdx.x * kRowElems,
-                             kRowElems * sizeof(cpx<float>));
-        // the owners' key loads go out first: their L2 latency overlaps the
-        // rotation, the digits and the forward transform
-        float4 kk[kRows][4];
+        for (; i < n; ++i) {
+            if (i > 0 && !mbar_wait_bounded(kfree, (uint32_t)(i - 1) & 1, abort)) {
+                gave_up();
+                break;
+            }
+            __syncwarp();
+            if (u == 0) mbar_arrive_expect_tx(kfull, (uint32_t)(Plan::kKeyParts * kHalf * sizeof(cpx<float>)));
+            __syncwarp();
+            if (u < Plan::kKeyParts)
+                bulk_copy_g2s(smem + Plan::key_off + (size_t)u * Plan::kKeyPart, src + (size_t)i * step_elems,
+                              (uint32_t)(kHalf * sizeof(cpx<float>)), kfull);
+            if (i + 2 < n && u < kRows)  // rows into L2 ahead of their copies
+                bulk_prefetch_l2(gsw + (size_t)(i + 2) * step_elems + (size_t)u * kRowElems,
+                                 kRowElems * sizeof(cpx<float>));
+        }
+        // no copy in flight at the end of the kernel
+        if (!mbar_wait_bounded(kfull, (uint32_t)(i - 1) & 1)) atomicExch(a.err, 3);
+        __syncwarp();
+    } else {
+        // barrier of all sets (the producer warp takes no part)
+        const auto step_sync = []() {
+            asm volatile("barrier.sync 15, %0;" ::"n"(kDuoThreads * Plan::kSets) : "memory");
+        };
+        const TwRegs<float> tw(hot_twiddles<float>(tables), t);
+        const DuoIdx ix = make_duo_idx(t, e);
+        cpx<float>* const xbuf[1] = {reinterpret_cast<cpx<float>*>(smem + Plan::x_off) + set * kDuoSlots};
+        const int bar_id = 1 + set;
+        const int halfBg = 1 << (kp.Bgbit - 1);
+        const uint32_t mask = (1u << kp.Bgbit) - 1;
+        const int decal = 32 - (lev + 1) * kp.Bgbit;
+        const int out_shift = e == 0 ? kp.split : 0;  // the high part counts 2^split
+        const float4* keys =
+            reinterpret_cast<const float4*>(smem + Plan::key_off + (size_t)(2 * set + e) * Plan::kKeyPart) + t;
+        uint32_t own[8] = {};  // owners: coefficients t + 64q (even lane) or 512 above (odd) of the output polynomial
         if (owner) {
 #pragma unroll
-            for (int p = 0; p < kRows; ++p) {
-                const float4* g4 =
-                    reinterpret_cast<const float4*>(step_keys + (size_t)p * kRowElems + (oj * 2 + opt) * kHalf);
-#pragma unroll
-                for (int qq = 0; qq < 4; ++qq) kk[p][qq] = __ldg(g4 + qq * 64 + t);
-            }
+            for (int q = 0; q < 8; ++q) own[q] = (uint32_t)acc[spread_word(set, t + 64 * q + e * kHalf)];
         }
-        cpx<float> v[8];
-        {
-            const int32_t* src = acc + jp * kN;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int x0 = t + 64 * r;
-                const uint32_t u0 = (uint32_t)rot_coef(src, x0, ai) - (uint32_t)src[x0] + kp.offset;
-                const uint32_t u1 =
-                    (uint32_t)rot_coef(src, x0 + kHalf, ai) - (uint32_t)src[x0 + kHalf] + kp.offset;
-                v[r] = digit_pair<float>(u0, u1, decal, mask, halfBg);
-            }
-        }
-        fft512_forward_ip1(v, sc.b0, tw, ix, t, bar_id);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) dsh[(g * 8 + q) * 64 + t] = v[q];
-        __syncthreads();  // every D written, every read of acc done
-        if (owner) {
-            cpx<float> o[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) o[q] = {0.f, 0.f};
-#pragma unroll
-            for (int p = 0; p < kRows; ++p)
-#pragma unroll
-                for (int qq = 0; qq < 4; ++qq) {
-                    const cpx<float> d0 = dsh[(p * 8 + 2 * qq) * 64 + t];
-                    const cpx<float> d1 = dsh[(p * 8 + 2 * qq + 1) * 64 + t];
-                    o[2 * qq] = cmac(o[2 * qq], d0, cpx<float>{kk[p][qq].x, kk[p][qq].y});
-                    o[2 * qq + 1] = cmac(o[2 * qq + 1], d1, cpx<float>{kk[p][qq].z, kk[p][qq].w});
+        const int32_t* bara = a.bara ? a.bara + (size_t)c * n : nullptr;
+        const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
+        const int32_t* rot = bara ? bara : xs;
+        int32_t rot_next = rot[0];
+#pragma unroll 1
+        for (int i = 0; i < n; ++i) {
+            const int ai = bara ? rot_next : mod_switch_2n(rot_next);
+            if (i + 1 < n) rot_next = rot[i + 1];
+            if (ai == 0) {  // tfhe_blindRotate_FFT.cpp:114 (uniform over the CTA): the keys go by unused
+                if (owner) {
+                    if (!mbar_wait_bounded(kfull, (uint32_t)i & 1, abort)) gave_up();
+                    __syncwarp();
+                    if ((threadIdx.x & 31) == 0) mbar_arrive(kfree);
                 }
-            fft512_inverse_ip1(o, sc.b0, tw, ix, t, bar_id);
-            uint32_t c0[8] = {}, c1[8] = {};  // the low part adds into them
-            round_part<float, 2>(o, opt, kp.split, c0, c1);
-            int32_t* dst = acc + oj * kN;
+                continue;
+            }
+            cpx<float> v[1][8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                const int x0 = t + 64 * q;
-                atomicAdd(reinterpret_cast<unsigned*>(dst + x0), c0[q]);
-                atomicAdd(reinterpret_cast<unsigned*>(dst + x0 + kHalf), c1[q]);
+                uint32_t u0, u1;
+                rotated_pair(acc, jp, t, q, ai, kp.offset, u0, u1);
+                v[0][q] = digit_pair<float>(u0, u1, decal, mask, halfBg);
             }
+            fft512_forward_duo<1>(v, xbuf, tw, ix, bar_id);
+            {
+                const int d0 = owner ? jp * Plan::kD + 2 * t + e : jp * Plan::kD + Plan::kDA + t;
+                const int dq = owner ? 128 : 64;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) dsh[d0 + dq * q] = v[0][q];
+            }
+            step_sync();  // every D in place; every read of acc done
+            if (owner) {
+                if (!mbar_wait_bounded(kfull, (uint32_t)i & 1, abort)) gave_up();
+                __syncwarp();
+                cpx<float> o[1][8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[0][q] = {0.f, 0.f};
+#pragma unroll
+                for (int qq = 0; qq < 4; ++qq)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        float4 w[L];
+#pragma unroll
+                        for (int lv = 0; lv < L; ++lv)
+                            w[lv] = keys[(j * L + lv) * 4 * (Plan::kKeyPart / 16) + qq * 64];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int q = 2 * qq + h;
+                            const cpx<float>* D = dsh + j * Plan::kD;
+                            const float4 da = reinterpret_cast<const float4*>(D)[q * 64 + t];
+                            o[0][q] = cmac(o[0][q], cpx<float>{da.x, da.y},
+                                           h ? cpx<float>{w[0].z, w[0].w} : cpx<float>{w[0].x, w[0].y});
+                            o[0][q] = cmac(o[0][q], cpx<float>{da.z, da.w},
+                                           h ? cpx<float>{w[1].z, w[1].w} : cpx<float>{w[1].x, w[1].y});
+                            if constexpr (L == 3)
+                                o[0][q] = cmac(o[0][q], D[Plan::kDA + q * 64 + t],
+                                               h ? cpx<float>{w[2].z, w[2].w} : cpx<float>{w[2].x, w[2].y});
+                        }
+                    }
+                __syncwarp();
+                if ((threadIdx.x & 31) == 0) mbar_arrive(kfree);
+                fft512_inverse_duo<1>(o, xbuf, tw, ix, bar_id);
+                // both parts through the wide rounding: for the high part (below
+                // 2^22) it gives round_small_pair's integer, and the lanes stay together
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    uint32_t c0, c1;
+                    round_wrap_pair(o[0][q], c0, c1);
+                    c0 <<= out_shift;
+                    c1 <<= out_shift;
+                    const uint32_t other = __shfl_xor_sync(0xffffffffu, e ? c0 : c1, 1);
+                    own[q] += (e ? c1 : c0) + other;
+                    spread_put(acc, set, t + 64 * q + e * kHalf, own[q]);
+                }
+            }
+            step_sync();  // the accumulator is updated before the next step reads it
         }
-        __syncthreads();  // the accumulator is updated before the next step reads it
     }
+    __syncthreads();
     if (a.acc_out) {
         int32_t* dst = a.acc_out + (size_t)c * 2 * kN;
-        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x) dst[i] = acc[i];
+        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x) dst[i] = acc[spread_word(i >> 10, i & (kN - 1))];
     }
     if (a.lwe_out) {
         // tLweExtractLweSample: a'_0 = a_0, a'_j = -a_{N-j}, b' = b_0
         int32_t* dst = a.lwe_out + (size_t)c * (kN + 1);
         for (int i = threadIdx.x; i < kN; i += blockDim.x)
-            dst[i] = i == 0 ? acc[0] : (int32_t)(0u - (uint32_t)acc[kN - i]);
-        if (threadIdx.x == 0) dst[kN] = acc[kN];
+            dst[i] = i == 0 ? acc[spread_word(0, 0)] : (int32_t)(0u - (uint32_t)acc[spread_word(0, kN - i)]);
+        if (threadIdx.x == 0) dst[kN] = acc[spread_word(1, 0)];
     }
 }
 
 // ----------------------------------------------------------------------
 // Blind rotation with one ciphertext over a cluster of two CTAs (two SMs).
 //
-// The spread kernel's work split across two SMs: CTA r of the cluster holds
+// The work of a step split across two SMs: CTA r of the cluster holds
 // accumulator polynomial r, runs the l forward transforms of polynomial r
 // (one per group) and owns output polynomial r (groups 0 and 1: the high and
 // the low key part).  Each group writes its transformed digits D_(r,lev) to
@@ -1271,8 +1383,7 @@ __global__ void __launch_bounds__(128 * L, 1) k_blind_rotate_spread(KParams kp, 
 // own mbarrier.  A push into buffer b at step k cannot overtake the peer's
 // reads of b at step k - 2: the pushing CTA has by then received the peer's
 // step k - 1 digits, which the peer sends only after its step k - 2
-// products.  Each SM carries half the spread kernel's shared-memory traffic
-// and transforms; the products are summed in the same order as every other
+// products.  The products are summed in the same order as every other
 // shape, so the ciphertexts are bit-identical to the spread kernel's.
 // Split-FP32 only, 1 CTA per SM (the shared-memory request is padded so
 // that the two CTAs take two SMs).
@@ -2607,7 +2718,7 @@ cudaError_t launch_spread(const DevParams& P, const Tables& T, const EpArgs& a, 
     auto kern = k_blind_rotate_spread<L>;
     cudaError_t e = set_smem(kern, Plan::total);
     if (e != cudaSuccess) return e;
-    kern<<<a.count, 128 * L, Plan::total, st>>>(kp, T, a);
+    kern<<<a.count, Plan::kThreads, Plan::total, st>>>(kp, T, a);
     return cudaGetLastError();
 }
 
@@ -2689,8 +2800,8 @@ cudaError_t launch_ring_pairs(const DevParams& P, const Tables& T, const EpArgs&
 // Measured per launch (default set): a wave of 6 per SM on
 // launch_ring_pairs 6.6 ms (138K gates/s), of 4 per SM on
 // launch_ring_batched 4.6 ms (132K/s), whatever the fill of the wave; the
-// spread kernel over a two-SM cluster 1.35 ms for up to one per two SMs;
-// the spread kernel 1.85 ms at 1 per SM (3.7 ms for two waves); the pair
+// spread kernel over a two-SM cluster 1.19 ms for up to one per two SMs;
+// the spread kernel 1.58 ms at 1 per SM (3.16 ms for two waves); the pair
 // kernel 2.6 ms at 1 per SM, 3.3 ms at 2, 5.1 ms at 3.  So: whole waves of
 // 6 per SM; a remainder of at most one per two SMs on the cluster spread
 // kernel, of at most 1 per SM on the spread kernel, of 2 per SM on the pair

@@ -630,6 +630,151 @@ __device__ __forceinline__ void fft512_inverse_ip1(cpx<R> (&v)[8], cpx<R>* x, co
     fft512_inverse_ip<1>(*reinterpret_cast<cpx<R>(*)[1][8]>(&v), xs, tw, ix, t, bar_id);
 }
 
+// ----------------------------------------------------------------------
+// Lane-pair forms: lanes 2t' and 2t'+1 of a warp hold the same points of two
+// transforms (two ciphertexts), so the two lanes of a pair read the same
+// twiddle and key words.  A 64- or 128-bit shared load whose adjacent lanes
+// read the same address takes half the wavefronts (measured: 1.06 / 2.06
+// clocks per warp load against 2.05 / 4.05; lanes 16 apart sharing an
+// address gain nothing).  128 threads per set of two transforms, thread
+// t = threadIdx / 2 of each.  The exchange slots interleave the two: point p
+// of transform `ct` lies at (p + p/8) * 2 + ct, which is free of bank
+// conflicts for all three access patterns (a half-warp's 8 points fall in 8
+// different slots mod 8) and a compile-time offset from one per-thread base
+// each.  In place, one 128-thread barrier per transform: pass B and C
+// exchange within 8 threads, that is 16 lanes of one warp.  The arithmetic
+// is that of fft512_forward_ip / fft512_inverse_ip, bit for bit.
+// ----------------------------------------------------------------------
+constexpr int kDuoThreads = 128;
+constexpr int kDuoSlots = 2 * kScratchStride;  // complex values of one exchange buffer (two transforms)
+
+// Per-thread slot bases of the three access patterns, in complex values.
+struct DuoIdx {
+    int a, b, c;
+};
+__device__ __forceinline__ DuoIdx make_duo_idx(int t, int ct) {
+    return {2 * spad(t) + ct, 2 * (72 * (t >> 3) + (t & 7)) + ct, 18 * t + ct};
+}
+// pattern A: point t + 64q; B: 64(t/8) + t%8 + 8r; C: 8t + r
+constexpr int kDuoA = 2 * 72, kDuoB = 2 * 9, kDuoC = 2;
+
+// A thread's twiddles psi^t W^(tq) and W^(8 (t%8) q): read from a table each
+// time, or held in registers from the start of the kernel (30 words, where
+// the registers allow: no table reads in the transform).
+template <typename R>
+struct TwTable {
+    const cpx<R>*pa, *pb;
+    __device__ __forceinline__ TwTable(const FftTwiddles<R>& tw, int t) : pa(tw.a + t), pb(tw.b + (t & 7)) {}
+    __device__ __forceinline__ cpx<R> a(int q) const { return pa[q * 64]; }
+    __device__ __forceinline__ cpx<R> b(int q) const { return pb[q * 8]; }
+};
+template <typename R>
+struct TwRegs {
+    cpx<R> va[8], vb[8];
+    __device__ __forceinline__ TwRegs(const FftTwiddles<R>& tw, int t) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            va[q] = tw.a[q * 64 + t];
+            vb[q] = tw.b[q * 8 + (t & 7)];
+        }
+    }
+    __device__ __forceinline__ cpx<R> a(int q) const { return va[q]; }
+    __device__ __forceinline__ cpx<R> b(int q) const { return vb[q]; }
+};
+
+// Barrier of a set, in the form that does not take the warp to be converged
+// (bar.sync does, and lanes leave the bounded waits one by one).
+__device__ __forceinline__ void duo_sync(int bar_id) {
+    asm volatile("barrier.sync %0, %1;" ::"r"(bar_id), "r"(kDuoThreads) : "memory");
+}
+
+template <int NB, typename R, typename Tw>
+__device__ __forceinline__ void fft512_forward_duo(cpx<R> (&v)[NB][8], cpx<R>* const (&x)[NB], const Tw& tw,
+                                                   const DuoIdx& ix, int bar_id) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+        for (int r = 1; r < 8; ++r) v[b][r] = cmul(v[b][r], twist_c<R>(r));
+        dft8<1>(v[b]);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const cpx<R> w = tw.a(q);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[b][q] = cmul(v[b][q], w);
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[b][ix.a + kDuoA * q] = v[b][q];
+    duo_sync(bar_id);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[b][r] = x[b][ix.b + kDuoB * r];
+        dft8<1>(v[b]);
+    }
+#pragma unroll
+    for (int q = 1; q < 8; ++q) {
+        const cpx<R> w = tw.b(q);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[b][q] = cmul(v[b][q], w);
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[b][ix.b + kDuoB * q] = v[b][q];
+    __syncwarp();
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[b][r] = x[b][ix.c + kDuoC * r];
+        dft8<1>(v[b]);
+    }
+}
+
+template <int NB, typename R, typename Tw>
+__device__ __forceinline__ void fft512_inverse_duo(cpx<R> (&v)[NB][8], cpx<R>* const (&x)[NB], const Tw& tw,
+                                                   const DuoIdx& ix, int bar_id) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        dft8<-1>(v[b]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[b][ix.c + kDuoC * q] = v[b][q];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (r == 0) {
+#pragma unroll
+            for (int b = 0; b < NB; ++b) v[b][0] = x[b][ix.b];
+        } else {
+            const cpx<R> w = tw.b(r);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) v[b][r] = cmulc(x[b][ix.b + kDuoB * r], w);
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        dft8<-1>(v[b]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[b][ix.b + kDuoB * q] = v[b][q];
+    }
+    duo_sync(bar_id);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const cpx<R> w = tw.a(r);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[b][r] = cmulc(x[b][ix.a + kDuoA * r], w);
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        dft8<-1>(v[b]);
+#pragma unroll
+        for (int q = 1; q < 8; ++q) v[b][q] = cmulc(v[b][q], twist_c<R>(q));
+    }
+}
+
 // Frequency held at (thread t, register q) after the forward transform.
 __host__ __device__ __forceinline__ int freq_of(int t, int q) {
     return (t >> 3) + 8 * (t & 7) + 64 * q;

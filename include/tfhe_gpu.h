@@ -115,10 +115,10 @@ size_t tfhe_gpu_device_bytes(const tfhe_gpu_ctx* ctx);
  *   10 = 6 per CTA on the same ring, transforms two at a time;
  *   11, 12, 13 = pair kernel: two 64-thread halves per ciphertext (about
  *       half the latency), 1, 2, 3 ciphertexts per CTA, shared ring;
- *   14 = spread kernel: one ciphertext over 2l groups of 64 threads; per
- *       step each group runs one forward transform, and four of them
- *       multiply all rows for one output part and transform it back (lowest
- *       latency), key rows from L2;
+ *   14 = spread kernel: one ciphertext per CTA over l sets of 128 threads,
+ *       two transforms each; two of the sets multiply all rows for one output
+ *       polynomial and transform it back (low latency up to one per SM), key
+ *       rows copied ahead by a producer warp;
  *   15 = automatic in fixed summation order: as 0, with the spread kernel
  *       (two waves) in place of the pair kernel, whose two halves' partial
  *       products round differently; every launch then sums the key rows in

@@ -81,6 +81,21 @@ def test_fp64_blind_rotate_from_accumulators(engines, torch_cuda, count):
     assert (_rotations(torch, e, "fp64", 0, acc, bara) == _rotations(torch, e, "fp64", 3, acc, bara)).all()
 
 
+# split-FP32, one per CTA: a few | one per SM and one more (a second wave)
+@pytest.mark.parametrize("params,count", [("default", 3), ("stress", 153)])
+def test_spread_kernel_matches_l2_direct(engines, torch_cuda, params, count):
+    torch = torch_cuda
+    e = engines(params)
+    x = _uniform(torch, count, count, e.params.n + 1)
+    x[0, 7] = 0
+    assert (_bootstraps(torch, e, "split_fp32", 14, x) == _bootstraps(torch, e, "split_fp32", 4, x)).all()
+    acc = _uniform(torch, 3, count, 2048)
+    bara = _uniform(torch, 4, count, e.params.n) & 2047
+    bara[:, 5] = 0
+    bara[0] = 0
+    assert (_rotations(torch, e, "split_fp32", 14, acc, bara) == _rotations(torch, e, "split_fp32", 4, acc, bara)).all()
+
+
 def _cur(torch):
     return torch.cuda.current_stream().cuda_stream
 
