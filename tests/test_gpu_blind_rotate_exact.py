@@ -96,6 +96,22 @@ def test_spread_kernel_matches_l2_direct(engines, torch_cuda, params, count):
     assert (_rotations(torch, e, "split_fp32", 14, acc, bara) == _rotations(torch, e, "split_fp32", 4, acc, bara)).all()
 
 
+# shape 0 over 1 to 2 per SM keeps the pair kernel's summation order (shape 12)
+# whatever runs it; shape 15, and shape 0 elsewhere, the order of the rows
+# (shape 4): edges of 1, 1.5, 2, 4, 4.5 and 5 per SM, and after a full wave
+@pytest.mark.parametrize("params,shape,count,like", [
+    ("stress", 0, 152, 4), ("stress", 0, 153, 12), ("default", 0, 228, 12), ("stress", 0, 229, 12),
+    ("default", 0, 304, 12), ("stress", 15, 153, 4), ("default", 15, 229, 4), ("stress", 0, 305, 4),
+    ("stress", 0, 609, 4), ("default", 0, 685, 4), ("stress", 0, 760, 4), ("stress", 0, 761, 4),
+    ("stress", 15, 912 + 160, 4), ("stress", 0, 912 + 650, 4)])
+def test_split_automatic_shape_keeps_its_summation_order(engines, torch_cuda, params, shape, count, like):
+    torch = torch_cuda
+    e = engines(params)
+    x = _uniform(torch, count, count, e.params.n + 1)
+    x[0, 9] = 0
+    assert (_bootstraps(torch, e, "split_fp32", shape, x) == _bootstraps(torch, e, "split_fp32", like, x)).all()
+
+
 def _cur(torch):
     return torch.cuda.current_stream().cuda_stream
 
