@@ -96,6 +96,23 @@ def test_spread_kernel_matches_l2_direct(engines, torch_cuda, params, count):
     assert (_rotations(torch, e, "split_fp32", 14, acc, bara) == _rotations(torch, e, "split_fp32", 4, acc, bara)).all()
 
 
+# split-FP32 in lane pairs, 6 and (l = 2) 4 per SM: one, an odd number in the last set, a whole wave and one more
+@pytest.mark.parametrize("params,shape,count", [("default", 10, 1), ("stress", 10, 911), ("default", 10, 913),
+                                                ("stress", 9, 3), ("stress", 9, 609)])
+def test_lane_pair_ring_matches_l2_direct(engines, torch_cuda, params, shape, count):
+    torch = torch_cuda
+    e = engines(params)
+    x = _uniform(torch, count, count, e.params.n + 1)
+    x[0, 7] = 0  # one of a pair stands still
+    assert (_bootstraps(torch, e, "split_fp32", shape, x) == _bootstraps(torch, e, "split_fp32", 4, x)).all()
+    if count < 10:
+        acc = _uniform(torch, 3, count, 2048)
+        bara = _uniform(torch, 4, count, e.params.n) & 2047
+        bara[:, 5] = 0
+        assert (_rotations(torch, e, "split_fp32", shape, acc, bara)
+                == _rotations(torch, e, "split_fp32", 4, acc, bara)).all()
+
+
 # shape 0 over 1 to 2 per SM keeps the pair kernel's summation order (shape 12)
 # whatever runs it; shape 15, and shape 0 elsewhere, the order of the rows
 # (shape 4): edges of 1, 1.5, 2, 4, 4.5 and 5 per SM, and after a full wave
