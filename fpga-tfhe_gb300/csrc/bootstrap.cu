@@ -1122,7 +1122,9 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
 // warp copies each step's key rows into shared memory (one 4 KB part of a row
 // a lane) as soon as the owners have used the last step's.  The products are
 // summed in the same order as in every other shape, so the ciphertexts are
-// the same bit for bit.
+// the same bit for bit; with PAIR, in the pair kernel's order: the rows of
+// each input polynomial on their own, then the two sums (for the batch sizes
+// that shape 0 has always run in that order).
 //
 // What bounds it: the shared-memory pipe (about 4,300 wavefronts of a step's
 // 5,200 clocks: the key values written and read 1,536, the transforms'
@@ -1182,7 +1184,7 @@ __device__ __forceinline__ void rotated_pair(const int32_t* acc, int j, int t, i
     r1 = ((uint32_t)w.y ^ m) - (uint32_t)p.y + (offset - m);
 }
 
-template <int L>
+template <int L, bool PAIR>
 __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spread(KParams kp, Tables T, EpArgs a) {
     using Plan = SpreadPlan<L>;
     constexpr int kRows = 2 * L;
@@ -1307,6 +1309,9 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
                 cpx<float> o[1][8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) o[0][q] = {0.f, 0.f};
+                cpx<float> other[8];  // PAIR: the rows of the other input polynomial apart
+#pragma unroll
+                for (int q = 0; q < 8; ++q) other[q] = {0.f, 0.f};
 #pragma unroll
                 for (int qq = 0; qq < 4; ++qq)
 #pragma unroll
@@ -1320,15 +1325,20 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
                             const int q = 2 * qq + h;
                             const cpx<float>* D = dsh + j * Plan::kD;
                             const float4 da = reinterpret_cast<const float4*>(D)[q * 64 + t];
-                            o[0][q] = cmac(o[0][q], cpx<float>{da.x, da.y},
-                                           h ? cpx<float>{w[0].z, w[0].w} : cpx<float>{w[0].x, w[0].y});
-                            o[0][q] = cmac(o[0][q], cpx<float>{da.z, da.w},
-                                           h ? cpx<float>{w[1].z, w[1].w} : cpx<float>{w[1].x, w[1].y});
+                            cpx<float>& z = PAIR && j == 1 ? other[q] : o[0][q];
+                            z = cmac(z, cpx<float>{da.x, da.y},
+                                     h ? cpx<float>{w[0].z, w[0].w} : cpx<float>{w[0].x, w[0].y});
+                            z = cmac(z, cpx<float>{da.z, da.w},
+                                     h ? cpx<float>{w[1].z, w[1].w} : cpx<float>{w[1].x, w[1].y});
                             if constexpr (L == 3)
-                                o[0][q] = cmac(o[0][q], D[Plan::kDA + q * 64 + t],
-                                               h ? cpx<float>{w[2].z, w[2].w} : cpx<float>{w[2].x, w[2].y});
+                                z = cmac(z, D[Plan::kDA + q * 64 + t],
+                                         h ? cpx<float>{w[2].z, w[2].w} : cpx<float>{w[2].x, w[2].y});
                         }
                     }
+                if constexpr (PAIR) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) o[0][q] = cadd(o[0][q], other[q]);
+                }
                 __syncwarp();
                 if ((threadIdx.x & 31) == 0) mbar_arrive(kfree);
                 fft512_inverse_duo<1>(o, xbuf, tw, ix, bar_id);
@@ -1384,7 +1394,8 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
 // reads of b at step k - 2: the pushing CTA has by then received the peer's
 // step k - 1 digits, which the peer sends only after its step k - 2
 // products.  The products are summed in the same order as every other
-// shape, so the ciphertexts are bit-identical to the spread kernel's.
+// shape, so the ciphertexts are bit-identical to the spread kernel's (and with
+// PAIR in the pair kernel's order, as there).
 // Split-FP32 only, 1 CTA per SM (the shared-memory request is padded so
 // that the two CTAs take two SMs).
 // ----------------------------------------------------------------------
@@ -1401,7 +1412,7 @@ struct Spread2Plan {
     static constexpr size_t request = total > 120 * 1024 ? total : 120 * 1024;  // one CTA per SM
 };
 
-template <int L>
+template <int L, bool PAIR>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
     k_blind_rotate_spread2(KParams kp, Tables T, EpArgs a) {
     static_assert(L >= 2, "two owner groups per CTA");
@@ -1507,9 +1518,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
             cpx<float> o[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) o[q] = {0.f, 0.f};
+            cpx<float> first[8];  // PAIR: polynomial 0's rows on their own
 #pragma unroll
             for (int p = 0; p < kRows; ++p) {
                 const int jp = p / L, lv = p - jp * L;
+                if (PAIR && p == L) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        first[q] = o[q];
+                        o[q] = {0.f, 0.f};
+                    }
+                }
                 const cpx<float>* D = jp == r ? dloc + lv * kHalf : drem + (buf * L + lv) * kHalf;
 #pragma unroll
                 for (int qq = 0; qq < 4; ++qq) {
@@ -1518,6 +1537,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
                     o[2 * qq] = cmac(o[2 * qq], d0, cpx<float>{kk[p][qq].x, kk[p][qq].y});
                     o[2 * qq + 1] = cmac(o[2 * qq + 1], d1, cpx<float>{kk[p][qq].z, kk[p][qq].w});
                 }
+            }
+            if constexpr (PAIR) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[q] = cadd(first[q], o[q]);
             }
             fft512_inverse_ip1(o, sc.b0, tw, ix, t, bar_id);
             uint32_t c0[8] = {}, c1[8] = {};  // the low part adds into them
@@ -2710,24 +2733,24 @@ cudaError_t launch_pair_t(const DevParams& P, const Tables& T, const EpArgs& a, 
     return cudaGetLastError();
 }
 
-template <int L>
+template <int L, bool PAIR = false>
 cudaError_t launch_spread(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
     if (a.count <= 0) return cudaSuccess;
     const KParams kp = make_kparams(P);
     using Plan = SpreadPlan<L>;
-    auto kern = k_blind_rotate_spread<L>;
+    auto kern = k_blind_rotate_spread<L, PAIR>;
     cudaError_t e = set_smem(kern, Plan::total);
     if (e != cudaSuccess) return e;
     kern<<<a.count, Plan::kThreads, Plan::total, st>>>(kp, T, a);
     return cudaGetLastError();
 }
 
-template <int L>
+template <int L, bool PAIR = false>
 cudaError_t launch_spread2(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
     if (a.count <= 0) return cudaSuccess;
     const KParams kp = make_kparams(P);
     using Plan = Spread2Plan<L>;
-    auto kern = k_blind_rotate_spread2<L>;
+    auto kern = k_blind_rotate_spread2<L, PAIR>;
     cudaError_t e = set_smem(kern, Plan::request);
     if (e != cudaSuccess) return e;
     kern<<<2 * a.count, 64 * L, Plan::request, st>>>(kp, T, a);
@@ -2796,39 +2819,55 @@ cudaError_t launch_ring_pairs(const DevParams& P, const Tables& T, const EpArgs&
     return launch_ring_t<float, 2, 6, L, true, 4, 2>(P, T, a, st);
 }
 
+// Up to two ciphertexts per SM: one per cluster of two SMs up to half as many
+// as SMs, one per CTA up to as many, and two launches (a wave of one per CTA,
+// then the rest) above.
+template <int L, bool PAIR>
+cudaError_t launch_low_latency(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
+    if (a.count <= kSmCount / 2) return launch_spread2<L, PAIR>(P, T, a, st);
+    const int rest = a.count - kSmCount;
+    if (rest <= 0 || rest > kSmCount / 2) return launch_spread<L, PAIR>(P, T, a, st);
+    const cudaError_t e = launch_spread<L, PAIR>(P, T, slice_blind_rotate(P, a, 0, kSmCount), st);
+    if (e != cudaSuccess) return e;
+    return launch_spread2<L, PAIR>(P, T, slice_blind_rotate(P, a, kSmCount, rest), st);
+}
+
 // Automatic shape of a split-FP32 blind rotation over `count` ciphertexts.
 // Measured per launch (default set): a wave of 6 per SM on
-// launch_ring_pairs 6.6 ms (138K gates/s), of 4 per SM on
-// launch_ring_batched 4.6 ms (132K/s), whatever the fill of the wave; the
-// spread kernel over a two-SM cluster 1.19 ms for up to one per two SMs;
-// the spread kernel 1.58 ms at 1 per SM (3.16 ms for two waves); the pair
-// kernel 2.6 ms at 1 per SM, 3.3 ms at 2, 5.1 ms at 3.  So: whole waves of
-// 6 per SM; a remainder of at most one per two SMs on the cluster spread
-// kernel, of at most 1 per SM on the spread kernel, of 2 per SM on the pair
-// kernel, of at most 4 per SM as one launch_ring_batched wave, else one
-// more 6-per-SM wave.
+// launch_ring_pairs 6.4 ms, of 4 per SM on launch_ring_batched 4.6 ms,
+// whatever the fill of the wave; the cluster kernel 1.19 ms for up to one
+// per two SMs; the spread kernel 1.58 ms at 1 per SM, 3.0 to 3.2 ms for two
+// waves.  So: whole waves of 6 per SM; a remainder of up to 2 per SM on those
+// two (2.7 ms up to 1.5 per SM, where the pair kernel took 3.24 ms for any
+// count of 2 per SM), of up to 4 per SM as one launch_ring_batched wave, of
+// up to 5 as that wave and the rest on the low-latency kernels (5.7 or 6.1
+// ms), else one more 6-per-SM wave.
 //
-// fixed_order (shape 15): the pair kernel, which adds its two halves' partial
-// products and so may round differently, is replaced by the spread kernel
-// (two waves for 2 per SM, 3.8 ms against 3.3 ms): every launch then sums
-// the 2l key rows in the same order, and a ciphertext's result does not
-// depend on the batch it runs in -- what a server that mixes requests needs.
+// A remainder of more than 1 and up to 2 per SM is summed in the pair
+// kernel's order, as it always was under shape 0.  fixed_order (shape 15):
+// every launch sums the 2l key rows in the same order, and a ciphertext's
+// result does not depend on the batch it runs in -- what a server that mixes
+// requests needs.
 template <int L>
 cudaError_t launch_auto_fp32(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st,
                              bool fixed_order = false) {
     const int wave = 6 * kSmCount;
     const int full = (a.count / wave) * wave;
     const int rest = a.count - full;
-    if (rest == 0 || rest > 4 * kSmCount) return launch_ring_pairs<L>(P, T, a, st);
+    if (rest == 0 || rest > 5 * kSmCount) return launch_ring_pairs<L>(P, T, a, st);
     if (full) {
         cudaError_t e = launch_ring_pairs<L>(P, T, slice_blind_rotate(P, a, 0, full), st);
         if (e != cudaSuccess) return e;
     }
     const EpArgs tail = slice_blind_rotate(P, a, full, rest);
-    if (rest > 2 * kSmCount) return launch_ring_batched<L>(P, T, tail, st);
-    if (rest > kSmCount && !fixed_order) return launch_pair_fp32<L>(P, T, tail, 2, st);
-    if (rest > kSmCount / 2) return launch_spread<L>(P, T, tail, st);
-    return launch_spread2<L>(P, T, tail, st);
+    if (rest > 2 * kSmCount) {
+        const int most = std::min(rest, 4 * kSmCount);
+        cudaError_t e = launch_ring_batched<L>(P, T, slice_blind_rotate(P, tail, 0, most), st);
+        if (e != cudaSuccess || most == rest) return e;
+        return launch_low_latency<L, false>(P, T, slice_blind_rotate(P, tail, most, rest - most), st);
+    }
+    if (rest > kSmCount && !fixed_order) return launch_low_latency<L, true>(P, T, tail, st);
+    return launch_low_latency<L, false>(P, T, tail, st);
 }
 
 // Automatic shape of an FP64 blind rotation.  Every shape gives the same
