@@ -216,13 +216,9 @@ __device__ __forceinline__ FftTwiddles<R> hot_twiddles(const cpx<R>* hot) {
 //                 L1 prefetch of the rows ahead of the transform;
 //   RingKeys   -- from a shared-memory ring filled by a producer warp with
 //                 bulk copies (see k_blind_rotate_ring).
-// FB digit polynomials are transformed together (fft512_forward_tw_multi), and
-// IB parts of an output polynomial are transformed back together.  IP: the
-// in-place transforms (fft512_forward_ip / fft512_inverse_ip: one group
-// barrier per transform instead of two), alternating the two exchange
-// buffers of each stream from one transform to the next.  EARLY: a block's
-// key rows are tested for arrival before its forward transforms and waited
-// for after them.
+// The l digit polynomials of an input polynomial are transformed together
+// (fft512_forward_tw_multi), and IB parts of an output polynomial are
+// transformed back together.
 // ----------------------------------------------------------------------
 template <typename R, int PARTS, int NB>
 struct StepCtx {
@@ -246,8 +242,6 @@ struct GlobalKeys {
             asm volatile("prefetch.global.L1 [%0];" ::"l"(gb + (size_t)ln * 128));
     }
     __device__ __forceinline__ const cpx<R>* acquire(int p) const { return gsw + (size_t)p * kRow; }
-    __device__ __forceinline__ bool poll(int) const { return true; }
-    __device__ __forceinline__ const cpx<R>* acquire_polled(int p, bool) const { return acquire(p); }
     __device__ __forceinline__ void release(int) const {}
     static constexpr bool kShared = false;
 };
@@ -285,48 +279,30 @@ __device__ __forceinline__ void mac_row(cpx<R> (&out)[2][PARTS][8], const cpx<R>
         }
 }
 
-// Levels lev0 .. lev0 + NBK - 1 of input polynomial jp: digits, NBK forward
-// transforms run together, and their key rows multiply-accumulated.
-template <int NBK, bool IP, bool EARLY, typename R, int PARTS, int NB, typename Keys>
+// The L levels of input polynomial jp: digits, forward transforms run
+// together, and their key rows multiply-accumulated.
+template <int L, typename R, int PARTS, int NB, typename Keys>
 __device__ __forceinline__ void forward_levels(const StepCtx<R, PARTS, NB>& S, Keys& keys,
                                                cpx<R> (&out)[2][PARTS][8], const uint32_t (&r0)[8],
-                                               const uint32_t (&r1)[8], int p0, int lev0, uint32_t mask,
-                                               int halfBg, int which) {
+                                               const uint32_t (&r1)[8], int p0, uint32_t mask, int halfBg) {
     const int t = S.t;
-    bool landed[NBK];
-#pragma unroll
-    for (int b = 0; b < NBK; ++b) landed[b] = EARLY ? keys.poll(p0 + lev0 + b) : false;
-    cpx<R> v[NBK][8];
+    cpx<R> v[L][8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
 #pragma unroll
-        for (int b = 0; b < NBK; ++b) {
-            const int decal = 32 - (lev0 + b + 1) * S.Bgbit;
-            v[b][r] = digit_pair<R>(r0[r], r1[r], decal, mask, halfBg);
-        }
+        for (int b = 0; b < L; ++b) v[b][r] = digit_pair<R>(r0[r], r1[r], 32 - (b + 1) * S.Bgbit, mask, halfBg);
     }
-    if constexpr (IP) {
-        cpx<R>* x[NBK];
+    fft512_forward_tw_multi<L>(v, *reinterpret_cast<const FftScratch<R>(*)[L]>(S.s), S.tw, S.ix, t, S.bar_id);
 #pragma unroll
-        for (int b = 0; b < NBK; ++b) x[b] = which ? S.s[b].b1 : S.s[b].b0;
-        fft512_forward_ip<NBK>(v, x, S.tw, S.ix, t, S.bar_id);
-    } else {
-        fft512_forward_tw_multi<NBK>(v, *reinterpret_cast<const FftScratch<R>(*)[NBK]>(S.s), S.tw, S.ix, t,
-                                     S.bar_id);
-    }
-#pragma unroll
-    for (int b = 0; b < NBK; ++b) {
-        const int p = p0 + lev0 + b;
-        mac_row<R, PARTS, Keys::kShared>(out, v[b], EARLY ? keys.acquire_polled(p, landed[b]) : keys.acquire(p),
-                                         t);
-        keys.release(p);
+    for (int b = 0; b < L; ++b) {
+        mac_row<R, PARTS, Keys::kShared>(out, v[b], keys.acquire(p0 + b), t);
+        keys.release(p0 + b);
     }
 }
 
-template <typename R, int PARTS, bool ROT, int L, int FB, int IB, int NB, bool IP = false, bool EARLY = false,
-          typename Keys>
+template <typename R, int PARTS, bool ROT, int L, int IB, int NB, typename Keys>
 __device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB>& S, Keys& keys, int a) {
-    static_assert(PARTS % IB == 0 && FB <= NB && IB <= NB, "batch sizes");
+    static_assert(PARTS % IB == 0 && L <= NB && IB <= NB, "batch sizes");
     const int t = S.t;
     const int halfBg = 1 << (S.Bgbit - 1);
     const uint32_t mask = (1u << S.Bgbit) - 1;
@@ -338,7 +314,6 @@ __device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB>& S, Keys& ke
         for (int pt = 0; pt < PARTS; ++pt)
 #pragma unroll
             for (int q = 0; q < 8; ++q) out[j][pt][q] = {(R)0, (R)0};
-    int which = 0;  // IP: the exchange buffer of the next transform
 
 #pragma unroll 1
     for (int jp = 0; jp < 2; ++jp) {
@@ -358,16 +333,7 @@ __device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB>& S, Keys& ke
             r0[r] += S.offset;
             r1[r] += S.offset;
         }
-        // blocks of FB levels, then the remaining L % FB together
-#pragma unroll
-        for (int lev0 = 0; lev0 + FB <= L; lev0 += FB) {
-            forward_levels<FB, IP, EARLY>(S, keys, out, r0, r1, jp * L, lev0, mask, halfBg, which);
-            which ^= 1;
-        }
-        if constexpr (L % FB != 0) {
-            forward_levels<L % FB, IP, EARLY>(S, keys, out, r0, r1, jp * L, L - L % FB, mask, halfBg, which);
-            which ^= 1;
-        }
+        forward_levels<L>(S, keys, out, r0, r1, jp * L, mask, halfBg);
     }
 
     // back to the coefficient domain (j unrolled: out[j] must stay in registers)
@@ -381,16 +347,8 @@ __device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB>& S, Keys& ke
             for (int b = 0; b < IB; ++b)
 #pragma unroll
                 for (int q = 0; q < 8; ++q) v[b][q] = out[j][pt0 + b][q];
-            if constexpr (IP) {
-                cpx<R>* x[IB];
-#pragma unroll
-                for (int b = 0; b < IB; ++b) x[b] = which ? S.s[b].b1 : S.s[b].b0;
-                fft512_inverse_ip<IB>(v, x, S.tw, S.ix, t, S.bar_id);
-            } else {
-                fft512_inverse_tw_multi<IB>(v, *reinterpret_cast<const FftScratch<R>(*)[IB]>(S.s), S.tw, S.ix,
-                                            t, S.bar_id);
-            }
-            which ^= 1;
+            fft512_inverse_tw_multi<IB>(v, *reinterpret_cast<const FftScratch<R>(*)[IB]>(S.s), S.tw, S.ix, t,
+                                        S.bar_id);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
 #pragma unroll
@@ -637,7 +595,7 @@ __global__ void __launch_bounds__(64 * GROUPS, 1) k_external_product(KParams kp,
             if (i + 1 < n) a_next = bara ? bara[i + 1] : mod_switch_2n(xs[i + 1]);
             if (ai == 0) continue;  // tfhe_blindRotate_FFT.cpp:114
             GlobalKeys<R, PARTS> keys{gsw_base + (size_t)i * gsw_elems};
-            ep_step<R, PARTS, true, L, L, PARTS, NB>(S, keys, ai);
+            ep_step<R, PARTS, true, L, PARTS, NB>(S, keys, ai);
         }
         if (a.acc_out) {
             int32_t* dst = a.acc_out + (size_t)c * 2 * kN;
@@ -660,10 +618,10 @@ __global__ void __launch_bounds__(64 * GROUPS, 1) k_external_product(KParams kp,
             group_sync(S.bar_id);
             GlobalKeys<R, PARTS> keys{reinterpret_cast<const cpx<R>*>(gsw + a.gsw_stride * (size_t)item)};
             if (MODE == kEpPlain) {
-                ep_step<R, PARTS, false, L, L, PARTS, NB>(S, keys, 0);
+                ep_step<R, PARTS, false, L, PARTS, NB>(S, keys, 0);
             } else {
                 const int ai = a.bara[item];
-                if (ai != 0) ep_step<R, PARTS, true, L, L, PARTS, NB>(S, keys, ai);
+                if (ai != 0) ep_step<R, PARTS, true, L, PARTS, NB>(S, keys, ai);
             }
             int32_t* dst = a.acc_out + (size_t)item * 2 * kN;
             for (int i = t; i < 2 * kN; i += 64) dst[i] = S.acc[i];
@@ -921,6 +879,13 @@ struct RingKeys {
             issue_one();
         }
     }
+    // Issue rows up to r + S - 1 whose slots are free, without waiting.
+    __device__ __forceinline__ void issue_ready(uint32_t r) {
+        while (next_issue < total && next_issue < r + S) {
+            if (next_issue >= S && !mbar_try_wait(&empty[next_issue % S], ((next_issue / S) - 1) & 1)) return;
+            issue_one();
+        }
+    }
     // Issue every row up to `last` (inclusive), waiting for their slots: used
     // before the producer blocks on another group, for rows that group needs.
     // Deadlock-free as long as the rows whose slots are reused (<= last - S)
@@ -949,31 +914,37 @@ struct RingKeys {
         if (!mbar_wait_bounded(&full[slot], (r / S) & 1, abort)) give_up();
         return ring + slot * kRow;
     }
-    // acquire() in two parts, so that the arrival test's round trip overlaps
-    // other work: poll() issues rows (producer) and tests once whether row p
-    // has landed; acquire_polled() waits (bounded) only if it had not.
+    __device__ __forceinline__ void release(int p) const { mbar_arrive(&empty[(row0 + (uint32_t)p) % S]); }
+};
+
+// The lane-pair kernel's way to the rows: acquire() in two parts, so that the
+// arrival test's round trip overlaps other work -- poll() issues rows whose
+// slots are free (producer, without waiting) and tests once whether row p has
+// landed, acquire_polled() issues and waits (bounded) only if it had not --
+// and one lane releases a slot for its whole warp (the slot's count is the
+// number of consumer warps).
+template <typename R, int PARTS, int S>
+struct PolledRingKeys : RingKeys<R, PARTS, S> {
+    using Base = RingKeys<R, PARTS, S>;
     __device__ __forceinline__ bool poll(int p) {
-        const uint32_t r = row0 + (uint32_t)p;
-        if (producer) issue_upto(r);
-        return mbar_try_wait(&full[r % S], (r / S) & 1);
+        const uint32_t r = this->row0 + (uint32_t)p;
+        if (this->producer) this->issue_ready(r);
+        __syncwarp();
+        return mbar_try_wait(&this->full[r % S], (r / S) & 1);
     }
     __device__ __forceinline__ const cpx<R>* acquire_polled(int p, bool landed) {
-        const uint32_t r = row0 + (uint32_t)p;
+        const uint32_t r = this->row0 + (uint32_t)p;
         const uint32_t slot = r % S;
-        if (!landed && !mbar_wait_bounded(&full[slot], (r / S) & 1, abort)) give_up();
-        return ring + slot * kRow;
-    }
-    // per_warp: one lane arrives for its whole warp once the warp has read
-    // the row (the slot's count is then the number of consumer warps); else
-    // every consumer thread arrives
-    bool per_warp;
-    __device__ __forceinline__ void release(int p) const {
-        if (per_warp) {
-            __syncwarp();
-            if ((threadIdx.x & 31) == 0) mbar_arrive(&empty[(row0 + (uint32_t)p) % S]);
-        } else {
-            mbar_arrive(&empty[(row0 + (uint32_t)p) % S]);
+        if (!landed) {
+            if (this->producer) this->issue_upto(r);
+            if (!mbar_wait_bounded(&this->full[slot], (r / S) & 1, this->abort)) this->give_up();
         }
+        __syncwarp();
+        return this->ring + slot * Base::kRow;
+    }
+    __device__ __forceinline__ void release(int p) const {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive(&this->empty[(this->row0 + (uint32_t)p) % S]);
     }
 };
 
@@ -990,22 +961,15 @@ struct RingPlan {
     static constexpr size_t total = group_off + GROUPS * group;
 };
 
-// NB = 1: one transform at a time (ep_step_lean).  NB > 1: the l forward
+// NB = 1: one transform at a time (ep_step_lean).  NB = l > 1: the l forward
 // and the PARTS inverse transforms of a step run together (ep_step), which
 // needs NB exchange buffer pairs per group and about 250 registers, so at
-// most four groups per CTA.  NB <= 2 uses the in-place transforms (one group
-// barrier per transform; measured faster), NB = 3 the two-barrier form (the
-// in-place form took its 608-gate wave from 4.57 to 4.90 ms).
+// most four groups per CTA.
 template <typename R, int PARTS, int GROUPS, int L, int S, bool INLINE, int NB = 1>
 __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
     k_blind_rotate_ring(KParams kp, Tables T, EpArgs a) {
     using Plan = RingPlan<R, PARTS, GROUPS, L, S, NB>;
     constexpr int kpl = 2 * L;
-    // measured on the two-at-a-time form (NB = 2), not faster for the others:
-    // one slot release per consumer warp (6.48 -> 6.45 ms per 912-gate wave)
-    // and the rows' arrival tested before the transforms (6.45 -> 6.41 ms;
-    // the 4-per-SM form went from 4.58 to 4.98 ms with it)
-    constexpr bool kPerWarp = NB == 2;
     extern __shared__ __align__(128) char smem[];
     cpx<R>* tables = reinterpret_cast<cpx<R>*>(smem);
     cpx<R>* ring = reinterpret_cast<cpx<R>*>(smem + Plan::ring_off);
@@ -1016,7 +980,7 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
     if (threadIdx.x == 0) {
         for (int i = 0; i < S; ++i) {
             mbar_init(&full[i], 1);
-            mbar_init(&empty[i], (kPerWarp ? 2 : 64) * active);
+            mbar_init(&empty[i], 64 * active);
         }
         *abort = 0;
         fence_mbar_init();
@@ -1028,7 +992,7 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
     const int n = kp.n;
     const uint32_t total_rows = (uint32_t)n * kpl;
     RingKeys<R, PARTS, S> keys{ring, full, empty, 0, a.err, abort, false,
-                               reinterpret_cast<const char*>(a.gsw), total_rows, 0, kPerWarp};
+                               reinterpret_cast<const char*>(a.gsw), total_rows, 0};
     if (!INLINE && warp == 2 * GROUPS) {
         // producer warp: one lane streams all n * 2l key rows in order
         if ((threadIdx.x & 31) == 0 && !a.stall_keys) {
@@ -1089,7 +1053,7 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
             continue;
         }
         if constexpr (NB == 1) ep_step_lean<R, PARTS, L>(St, keys, ai);
-        else ep_step<R, PARTS, true, L, (NB < L ? NB : L), PARTS, NB, (NB <= 2), kPerWarp>(St, keys, ai);
+        else ep_step<R, PARTS, true, L, PARTS, NB>(St, keys, ai);
     }
     if (keys.producer) keys.drain();
     if (a.acc_out) {
@@ -1101,6 +1065,247 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
         for (int i = t; i < kN; i += 64)
             dst[i] = i == 0 ? St.acc[0] : (int32_t)(0u - (uint32_t)St.acc[kN - i]);
         if (t == 0) dst[kN] = St.acc[kN];
+    }
+}
+
+// ----------------------------------------------------------------------
+// The throughput kernel: the shared key ring with ciphertexts in lane pairs.
+//
+// A set of 128 threads runs two ciphertexts: lanes 2t' and 2t'+1 hold the
+// same transform points of the two (fft512_forward_duo), so their twiddle and
+// key-row loads share addresses within a lane pair and take half the
+// shared-memory wavefronts.  FB levels are transformed together, then the
+// remaining l % FB, and the two key parts of an output together.
+//
+// Accumulators of a set lie as [polynomial][x < 512][ct] pairs of words
+// (coefficients x and x + 512): a thread's rotated read of a folded point is
+// one 64-bit load, whose pair of words the rotation by a leaves together
+// (swapped when (x - a) mod 1024 >= 512), and two ciphertexts with different
+// a fall on different banks (even and odd 64-bit units).
+//
+// A step with a_i = 0 runs as an exact no-op instead of being skipped (every
+// digit is 0), so the set's barrier and the ring stay in step whatever the
+// other ciphertext does.  In a set with one ciphertext left the other lane
+// of each pair repeats it and stores nothing.
+//
+// What bounds it: the FP32 pipe and the register file's operand reads
+// together with the latency of 12 warps per SM (FMA pipe 52 %, issue 54 %,
+// shared-memory pipe 64 %).  Against one ciphertext per 64 threads, which was
+// at 80 % of the shared-memory pipe (key rows and twiddles 1,130 of 2,750
+// wavefronts per ciphertext and step): 6.41 -> 6.23 ms for 912 ciphertexts of
+// the default set, 4.03 -> 3.88 ms for l = 2.  Eight per SM with transforms
+// one at a time took 8.5 ms for 1,216; unrolling over the two input
+// polynomials 10.5 ms (the code no longer fits the instruction cache).
+// ----------------------------------------------------------------------
+template <int SETS, int L, int S, int NB>
+struct DuoPlan {
+    static constexpr size_t kRowBytes = (size_t)2 * 2 * kHalf * sizeof(cpx<float>);
+    static constexpr size_t ring_off = (kHotSize * sizeof(cpx<float>) + 127) & ~(size_t)127;
+    static constexpr size_t bar_off = ring_off + S * kRowBytes;
+    static constexpr size_t flag_off = bar_off + 2 * S * sizeof(uint64_t);
+    static constexpr size_t set_off = (flag_off + sizeof(int) + 127) & ~(size_t)127;
+    static constexpr size_t acc = 2 * 2 * kN * sizeof(int32_t);
+    static constexpr size_t set = acc + NB * 2 * kDuoSlots * sizeof(cpx<float>);
+    static constexpr size_t total = set_off + SETS * set;
+};
+
+// word of coefficient x of polynomial j of ciphertext ct of a set
+__device__ __forceinline__ int duo_word(int j, int x, int ct) {
+    return j * 2 * kN + (((x & (kHalf - 1)) << 1) + ct) * 2 + (x >> 9);
+}
+
+struct DuoCtx {
+    TwTable<float> tw;
+    DuoIdx ix;
+    cpx<float>* s;  // exchange buffers, two per transform of a block
+    int32_t* acc;
+    int t, ct, bar_id;
+    int Bgbit, split;
+    uint32_t offset;
+};
+
+// out[j][pt] += v * key row, point by point so that the four products of one
+// point come one after another: v[q] is then the same register operand of
+// eight packed FMAs in a row.  A packed FMA with three different register
+// pairs takes 3 clocks (operand reads), with one reused 2.1 to 2.4; this
+// order is 0.11 ms of the 6.23.
+__device__ __forceinline__ void duo_mac_row(cpx<float> (&out)[2][2][8], const cpx<float> (&v)[8],
+                                            const cpx<float>* __restrict__ g, int t) {
+    const float4* g4 = reinterpret_cast<const float4*>(g) + t;
+#pragma unroll
+    for (int qq = 0; qq < 4; ++qq) {
+        float4 w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = g4[u * (kHalf / 2) + qq * 64];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int q = 2 * qq + e;
+            float2 o[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                o[u] = __ffma2_rn(pk(v[q]), bc(e ? w[u].z : w[u].x), pk(out[u >> 1][u & 1][q]));
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                out[u >> 1][u & 1][q] = unpk(__ffma2_rn(times_i(v[q]), bc(e ? w[u].w : w[u].y), o[u]));
+        }
+    }
+}
+
+template <int NBK, typename Keys>
+__device__ __forceinline__ void duo_levels(const DuoCtx& S, Keys& keys, cpx<float> (&out)[2][2][8],
+                                           const uint32_t (&r0)[8], const uint32_t (&r1)[8], int p0, int lev0,
+                                           int which) {
+    const uint32_t mask = (1u << S.Bgbit) - 1;
+    const int halfBg = 1 << (S.Bgbit - 1);
+    bool landed[NBK];
+#pragma unroll
+    for (int b = 0; b < NBK; ++b) landed[b] = keys.poll(p0 + lev0 + b);
+    cpx<float> v[NBK][8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int b = 0; b < NBK; ++b)
+            v[b][r] = digit_pair<float>(r0[r], r1[r], 32 - (lev0 + b + 1) * S.Bgbit, mask, halfBg);
+    cpx<float>* x[NBK];
+#pragma unroll
+    for (int b = 0; b < NBK; ++b) x[b] = S.s + (2 * b + which) * kDuoSlots;
+    fft512_forward_duo<NBK>(v, x, S.tw, S.ix, S.bar_id);
+#pragma unroll
+    for (int b = 0; b < NBK; ++b) {
+        const int p = p0 + lev0 + b;
+        duo_mac_row(out, v[b], keys.acquire_polled(p, landed[b]), S.t);
+        keys.release(p);
+    }
+}
+
+template <int L, int FB, typename Keys>
+__device__ __forceinline__ void duo_step(const DuoCtx& S, Keys& keys, int a) {
+    const int t = S.t;
+    cpx<float> out[2][2][8];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int pt = 0; pt < 2; ++pt)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) out[j][pt][q] = {0.f, 0.f};
+    int which = 0;  // the exchange buffers of the next transforms (in-place form: alternating)
+
+#pragma unroll 1
+    for (int jp = 0; jp < 2; ++jp) {
+        const int2* src = reinterpret_cast<const int2*>(S.acc + jp * 2 * kN) + S.ct;
+        uint32_t r0[8], r1[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int s = t + 64 * r - a;
+            const int2 w = src[(s & (kHalf - 1)) * 2];
+            const int2 p = src[(t + 64 * r) * 2];
+            // coefficient x reads s mod 1024, negated when s mod 2048 >= 1024; x + 512 reads s + 512
+            const uint32_t w0 = (uint32_t)(s & kHalf ? w.y : w.x), w1 = (uint32_t)(s & kHalf ? w.x : w.y);
+            r0[r] = S.offset - (uint32_t)p.x + (s & kN ? 0u - w0 : w0);
+            r1[r] = S.offset - (uint32_t)p.y + ((s + kHalf) & kN ? 0u - w1 : w1);
+        }
+#pragma unroll
+        for (int lev0 = 0; lev0 + FB <= L; lev0 += FB) {
+            duo_levels<FB>(S, keys, out, r0, r1, jp * L, lev0, which);
+            which ^= 1;
+        }
+        if constexpr (L % FB != 0) {
+            duo_levels<L % FB>(S, keys, out, r0, r1, jp * L, L - L % FB, which);
+            which ^= 1;
+        }
+    }
+
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        cpx<float>* const x[2] = {S.s + which * kDuoSlots, S.s + (2 + which) * kDuoSlots};
+        fft512_inverse_duo<2>(out[j], x, S.tw, S.ix, S.bar_id);
+        which ^= 1;
+        int2* dst = reinterpret_cast<int2*>(S.acc + j * 2 * kN) + S.ct;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            uint32_t h0, h1, l0, l1;
+            round_small_pair(out[j][0][q], h0, h1);
+            round_wrap_pair(out[j][1][q], l0, l1);
+            int2 w = dst[(t + 64 * q) * 2];
+            w.x = (int32_t)((uint32_t)w.x + (h0 << S.split) + l0);
+            w.y = (int32_t)((uint32_t)w.y + (h1 << S.split) + l1);
+            dst[(t + 64 * q) * 2] = w;
+        }
+    }
+    duo_sync(S.bar_id);
+}
+
+template <int SETS, int L, int S, int FB>
+__global__ void __launch_bounds__(kDuoThreads * SETS, 1) k_blind_rotate_duo(KParams kp, Tables T, EpArgs a) {
+    constexpr int NB = 2;
+    static_assert(FB <= NB && FB <= L, "buffers for the forward block and both parts");
+    using Plan = DuoPlan<SETS, L, S, NB>;
+    constexpr int kpl = 2 * L;
+    extern __shared__ __align__(128) char smem[];
+    cpx<float>* tables = reinterpret_cast<cpx<float>*>(smem);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + Plan::bar_off);
+    uint64_t* empty = full + S;
+    volatile int* abort = reinterpret_cast<volatile int*>(smem + Plan::flag_off);
+    const int left = a.count - (int)blockIdx.x * 2 * SETS;  // ciphertexts from this CTA on
+    const int active = min(SETS, (left + 1) >> 1);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < S; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 4 * active);  // one release per consumer warp
+        }
+        *abort = 0;
+        fence_mbar_init();
+    }
+    load_hot_tables<float>(tables, T);
+    __syncthreads();
+
+    const int set = threadIdx.x >> 7;
+    if (set >= active) return;
+    const int ct = threadIdx.x & 1, t = (threadIdx.x & 127) >> 1;
+    const bool live = 2 * set + ct < left;
+    const int c = blockIdx.x * 2 * SETS + 2 * set + (live ? ct : 0);
+    const int n = kp.n;
+    PolledRingKeys<float, 2, S> keys{{reinterpret_cast<cpx<float>*>(smem + Plan::ring_off), full, empty, 0, a.err, abort,
+                                      threadIdx.x == 0 && !a.stall_keys, reinterpret_cast<const char*>(a.gsw),
+                                      (uint32_t)n * kpl, 0}};
+    char* sbase = smem + Plan::set_off + (size_t)set * Plan::set;
+    const DuoCtx St{TwTable<float>(hot_twiddles<float>(tables), t), make_duo_idx(t, ct),
+                    reinterpret_cast<cpx<float>*>(sbase + Plan::acc), reinterpret_cast<int32_t*>(sbase), t, ct, 1 + set,
+                    kp.Bgbit, kp.split, kp.offset};
+
+    if (a.acc_in) {
+        const int32_t* src = a.acc_in + (size_t)c * 2 * kN;
+        for (int i = t; i < 2 * kN; i += 64) St.acc[duo_word(i >> 10, i & (kN - 1), ct)] = src[i];
+    } else {
+        const int barb = mod_switch_2n(a.x[(size_t)c * (n + 1) + n]);
+        for (int i = t; i < kN; i += 64) {
+            St.acc[duo_word(0, i, ct)] = 0;
+            St.acc[duo_word(1, i, ct)] = test_vector_coef(a, c, barb, i);
+        }
+    }
+    duo_sync(St.bar_id);
+    const int32_t* bara = a.bara ? a.bara + (size_t)c * n : nullptr;
+    const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
+    int a_next = bara ? bara[0] : mod_switch_2n(xs[0]);
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+        const int ai = a_next;
+        if (i + 1 < n) a_next = bara ? bara[i + 1] : mod_switch_2n(xs[i + 1]);
+        keys.row0 = (uint32_t)i * kpl;
+        duo_step<L, FB>(St, keys, ai);
+    }
+    if (keys.producer) keys.drain();
+    if (!live) return;
+    if (a.acc_out) {
+        int32_t* dst = a.acc_out + (size_t)c * 2 * kN;
+        for (int i = t; i < 2 * kN; i += 64) dst[i] = St.acc[duo_word(i >> 10, i & (kN - 1), ct)];
+    }
+    if (a.lwe_out) {
+        // tLweExtractLweSample: a'_0 = a_0, a'_j = -a_{N-j}, b' = b_0
+        int32_t* dst = a.lwe_out + (size_t)c * (kN + 1);
+        for (int i = t; i < kN; i += 64)
+            dst[i] = i == 0 ? St.acc[duo_word(0, 0, ct)] : (int32_t)(0u - (uint32_t)St.acc[duo_word(0, kN - i, ct)]);
+        if (t == 0) dst[kN] = St.acc[duo_word(1, 0, ct)];
     }
 }
 
@@ -2166,7 +2371,7 @@ __global__ void __launch_bounds__(128 * L, 1) k_blind_rotate_spread_f64(KParams 
 // as k_blind_rotate_ring; each row is read by one half of every ciphertext.
 // ----------------------------------------------------------------------
 __device__ __forceinline__ void pair_sync(int bar_id) {
-    asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(2 * kFftThreads) : "memory");
+    asm volatile("barrier.sync %0, %1;" ::"r"(bar_id), "r"(2 * kFftThreads) : "memory");
 }
 
 // h is the half; out[h] and out[1 - h] are picked by uniform branches so
@@ -2300,7 +2505,7 @@ __global__ void __launch_bounds__(128 * PAIRS, 1) k_blind_rotate_pair(KParams kp
     if (pr >= active) return;
     const int n = kp.n;
     RingKeys<R, PARTS, S> keys{ring, full, empty, 0, a.err, abort, threadIdx.x == 0 && !a.stall_keys,
-                               reinterpret_cast<const char*>(a.gsw), (uint32_t)n * kpl, 0, false};
+                               reinterpret_cast<const char*>(a.gsw), (uint32_t)n * kpl, 0};
 
     char* pbase = smem + Plan::pair_off + (size_t)pr * Plan::pair;
     StepCtx<R, PARTS, 1> St;
@@ -2807,16 +3012,31 @@ cudaError_t launch_pair_fp32(const DevParams& P, const Tables& T, const EpArgs& 
     return launch_pair_t<float, 2, 3, L, 4>(P, T, a, st);
 }
 
-// Batched ring kernels: 4 per CTA with a step's l forward transforms run
-// together (250 registers, 8 warps per SM), or 6 per CTA with transforms two
-// at a time (168 registers, 12 warps per SM).
+template <int SETS, int L>
+cudaError_t launch_duo(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
+    if (a.count <= 0) return cudaSuccess;
+    const KParams kp = make_kparams(P);
+    using Plan = DuoPlan<SETS, L, 4, 2>;
+    auto kern = k_blind_rotate_duo<SETS, L, 4, 2>;
+    cudaError_t e = set_smem(kern, Plan::total);
+    if (e != cudaSuccess) return e;
+    kern<<<(a.count + 2 * SETS - 1) / (2 * SETS), kDuoThreads * SETS, Plan::total, st>>>(kp, T, a);
+    return cudaGetLastError();
+}
+
+// Batched ring kernels: 4 per CTA (8 warps per SM) -- for l = 3 with a step's
+// three forward transforms run together in one ciphertext's 64 threads (4.56
+// ms for 608; in lane pairs two at a time 4.71 ms), for l = 2 in lane pairs
+// (2.79 ms against 2.90) -- or 6 per CTA in lane pairs, transforms two at a
+// time (168 registers, 12 warps per SM).
 template <int L>
 cudaError_t launch_ring_batched(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
-    return launch_ring_t<float, 2, 4, L, true, 4, (L > 2 ? L : 2)>(P, T, a, st);
+    if constexpr (L == 2) return launch_duo<2, L>(P, T, a, st);
+    else return launch_ring_t<float, 2, 4, L, true, 4, L>(P, T, a, st);
 }
 template <int L>
 cudaError_t launch_ring_pairs(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
-    return launch_ring_t<float, 2, 6, L, true, 4, 2>(P, T, a, st);
+    return launch_duo<3, L>(P, T, a, st);
 }
 
 // Up to two ciphertexts per SM: one per cluster of two SMs up to half as many
@@ -2834,7 +3054,7 @@ cudaError_t launch_low_latency(const DevParams& P, const Tables& T, const EpArgs
 
 // Automatic shape of a split-FP32 blind rotation over `count` ciphertexts.
 // Measured per launch (default set): a wave of 6 per SM on
-// launch_ring_pairs 6.4 ms, of 4 per SM on launch_ring_batched 4.6 ms,
+// launch_ring_pairs 6.2 ms, of 4 per SM on launch_ring_batched 4.6 ms,
 // whatever the fill of the wave; the cluster kernel 1.19 ms for up to one
 // per two SMs; the spread kernel 1.58 ms at 1 per SM, 3.0 to 3.2 ms for two
 // waves.  So: whole waves of 6 per SM; a remainder of up to 2 per SM on those
