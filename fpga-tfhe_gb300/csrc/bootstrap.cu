@@ -1673,8 +1673,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
     const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
     const int32_t* rot = bara ? bara : xs;
     int32_t rot_next = rot[0];
-    if (threadIdx.x < kRows && (threadIdx.x & 1) == r)
-        bulk_prefetch_l2(gsw + (size_t)threadIdx.x * kRowElems, kRowElems * sizeof(cpx<float>));
+    // side jobs of the last warp, done once its group's digits are out: with
+    // l = 3 that group owns no output (they cost a warp 230 clocks a step)
+    const int side = (int)threadIdx.x - (64 * L - 32);
+    const auto prefetch_rows = [&](int step) {
+        if (step < n && side >= 0 && side < kRows && (side & 1) == r)
+            bulk_prefetch_l2(gsw + (size_t)step * step_elems + (size_t)side * kRowElems,
+                             kRowElems * sizeof(cpx<float>));
+    };
+    // a step's incoming digits: one arrival and l x 4 KB of stores
+    const auto expect_digits = [&](int b) {
+        if (side == 0) mbar_arrive_expect_tx(&dbar[b], (uint32_t)(L * kHalf * sizeof(cpx<float>)));
+    };
+    prefetch_rows(0);
+    prefetch_rows(1);
+    expect_digits(0);
     uint32_t k = 0;  // steps taken (the same in both CTAs)
 #pragma unroll 1
     for (int i = 0; i < n; ++i) {
@@ -1682,22 +1695,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
         if (i + 1 < n) rot_next = rot[i + 1];
         if (ai == 0) continue;  // tfhe_blindRotate_FFT.cpp:114 (uniform over the cluster)
         const int buf = (int)(k & 1);
-        // this step's incoming digits: one arrival and l x 4 KB of stores
-        if (threadIdx.x == 0) mbar_arrive_expect_tx(&dbar[buf], (uint32_t)(L * kHalf * sizeof(cpx<float>)));
         const cpx<float>* step_keys = gsw + (size_t)i * step_elems;
-        if (i + 1 < n && threadIdx.x < kRows && (threadIdx.x & 1) == r)  // next step's rows into L2
-            bulk_prefetch_l2(step_keys + step_elems + (size_t)threadIdx.x * kRowElems,
-                             kRowElems * sizeof(cpx<float>));
-        float4 kk[kRows][4];
-        if (owner) {  // part (r, opt) of every row, issued before the transform
-#pragma unroll
-            for (int p = 0; p < kRows; ++p) {
-                const float4* g4 =
-                    reinterpret_cast<const float4*>(step_keys + (size_t)p * kRowElems + (r * 2 + opt) * kHalf);
-#pragma unroll
-                for (int qq = 0; qq < 4; ++qq) kk[p][qq] = __ldg(g4 + qq * 64 + t);
-            }
-        }
         cpx<float> v[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -1714,7 +1712,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
             st_async_f2(drem_peer + (uint32_t)((buf * L * kHalf + e) * sizeof(cpx<float>)), v[q].x, v[q].y,
                         dbar_peer + (uint32_t)(buf * sizeof(uint64_t)));
         }
+        // the owners' key values, part (r, opt) of every row, loaded while the
+        // peer's digits travel: 96 16-byte loads a step and SM hold the
+        // load/store unit some 500 clocks, which the rotation and the
+        // transform would wait for (1.184 -> 1.119 ms against loads at the
+        // start of the step)
+        float4 kk[kRows][4];
+        if (owner) {
+#pragma unroll
+            for (int p = 0; p < kRows; ++p) {
+                const float4* g4 =
+                    reinterpret_cast<const float4*>(step_keys + (size_t)p * kRowElems + (r * 2 + opt) * kHalf);
+#pragma unroll
+                for (int qq = 0; qq < 4; ++qq) kk[p][qq] = __ldg(g4 + qq * 64 + t);
+            }
+        }
         __syncthreads();  // every local D in place; every read of acc done
+        prefetch_rows(i + 2);
+        expect_digits(buf ^ 1);  // the other buffer's last digits were used a step ago
         if (owner) {
             if (!mbar_wait_cluster_bounded(&dbar[buf], (k >> 1) & 1, abort)) {  // the peer's D landed
                 *abort = 1;
@@ -3055,7 +3070,7 @@ cudaError_t launch_low_latency(const DevParams& P, const Tables& T, const EpArgs
 // Automatic shape of a split-FP32 blind rotation over `count` ciphertexts.
 // Measured per launch (default set): a wave of 6 per SM on
 // launch_ring_pairs 6.2 ms, of 4 per SM on launch_ring_batched 4.6 ms,
-// whatever the fill of the wave; the cluster kernel 1.19 ms for up to one
+// whatever the fill of the wave; the cluster kernel 1.12 ms for up to one
 // per two SMs; the spread kernel 1.58 ms at 1 per SM, 3.0 to 3.2 ms for two
 // waves.  So: whole waves of 6 per SM; a remainder of up to 2 per SM on those
 // two (2.7 ms up to 1.5 per SM, where the pair kernel took 3.24 ms for any

@@ -128,7 +128,7 @@ size_t tfhe_gpu_device_bytes(const tfhe_gpu_ctx* ctx);
  *       holds one accumulator polynomial, runs its l forward transforms and
  *       owns its output polynomial; transformed digits cross SMs as
  *       asynchronous stores into the peer's shared memory, counted on its
- *       mbarrier (lowest latency: about 1.33 ms for a single gate's blind
+ *       mbarrier (lowest latency: about 1.12 ms for a single gate's blind
  *       rotation).
  * FP64: 0 = automatic (the default): whole waves of three ciphertexts per SM
  * on 3; a remainder of up to 48 on an eight-SM cluster kernel, of up to one
