@@ -106,6 +106,20 @@ tfhe_gpu_status check_device_status(tfhe_gpu_ctx* ctx) {
     return fail(ctx, TFHE_GPU_TIMEOUT, "a bounded wait in a kernel gave up (key-row ring stalled)");
 }
 
+// The end of a host-buffer call: `bytes` of results at d_out to `out`, the
+// status word with them, one wait for both.  Results that fit the staging
+// buffer pass through it (a copy into pageable memory waits by itself).
+tfhe_gpu_status finish_host_call(tfhe_gpu_ctx* ctx, void* out, const void* d_out, size_t bytes, cudaStream_t st) {
+    const bool staged = bytes + 16 <= tfhe_gpu_ctx::kStageBytes;
+    volatile int32_t* status = reinterpret_cast<int32_t*>(ctx->h_stage);
+    char* results = staged ? ctx->h_stage + 16 : static_cast<char*>(out);
+    CK(ctx, cudaMemcpyAsync(ctx->h_stage, ctx->d_err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    CK(ctx, cudaMemcpyAsync(results, d_out, bytes, cudaMemcpyDeviceToHost, st));
+    CK(ctx, cudaStreamSynchronize(st));
+    if (staged) std::memcpy(out, results, bytes);
+    return *status == 0 ? TFHE_GPU_OK : check_device_status(ctx);
+}
+
 tfhe_gpu_status need_bk(tfhe_gpu_ctx* ctx, int32_t form) {
     if (!form_ok(form)) return fail(ctx, TFHE_GPU_BAD_PARAM, "unknown form");
     if (!ctx->d_bk[form]) return fail(ctx, TFHE_GPU_NO_KEY, "bootstrapping key of this form not uploaded");
@@ -265,6 +279,7 @@ tfhe_gpu_status tfhe_gpu_create(const tfhe_params* params, int32_t device, tfhe_
     ctx->key_bytes = b64 + b32;
     if (cudaMalloc(&ctx->d_err, sizeof(int32_t)) != cudaSuccess) return bail(TFHE_GPU_OOM);
     if (cudaMemset(ctx->d_err, 0, sizeof(int32_t)) != cudaSuccess) return bail(TFHE_GPU_DEVICE_ERROR);
+    if (cudaMallocHost(&ctx->h_stage, tfhe_gpu_ctx::kStageBytes) != cudaSuccess) return bail(TFHE_GPU_OOM);
     *out = ctx;
     return TFHE_GPU_OK;
 }
@@ -282,6 +297,7 @@ void tfhe_gpu_destroy(tfhe_gpu_ctx* ctx) {
         if (ctx->d_scratch[s]) cudaFree(ctx->d_scratch[s]);
     if (ctx->d_tables) cudaFree(ctx->d_tables);
     if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->side) cudaStreamDestroy(ctx->side);
@@ -722,20 +738,28 @@ tfhe_gpu_status tfhe_gpu_bootsGates_host(tfhe_gpu_ctx* ctx, const int32_t* gates
     if (count == 0) return TFHE_GPU_OK;
     const size_t w = (size_t)ctx->P.n + 1;
     const size_t lwe_bytes = (size_t)count * w * sizeof(int32_t);
-    void *d_io = nullptr, *d_g = nullptr;
-    RET(ensure_scratch(ctx, 3, 3 * lwe_bytes + (gates ? count * sizeof(int32_t) : 0), &d_io));
+    const size_t gate_bytes = gates ? count * sizeof(int32_t) : 0;
+    void* d_io = nullptr;
+    RET(ensure_scratch(ctx, 3, 3 * lwe_bytes + gate_bytes, &d_io));
     int32_t* d_ca = (int32_t*)d_io;
     int32_t* d_cb = d_ca + (size_t)count * w;
-    int32_t* d_out = d_cb + (size_t)count * w;
-    if (gates) d_g = d_out + (size_t)count * w;
+    int32_t* d_g = gates ? d_cb + (size_t)count * w : nullptr;
+    int32_t* d_out = d_cb + (size_t)count * w + (gates ? count : 0);
     cudaStream_t st = ctx->stream;
-    CK(ctx, cudaMemcpyAsync(d_ca, ca, lwe_bytes, cudaMemcpyHostToDevice, st));
-    CK(ctx, cudaMemcpyAsync(d_cb, cb, lwe_bytes, cudaMemcpyHostToDevice, st));
-    if (gates) CK(ctx, cudaMemcpyAsync(d_g, gates, count * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    RET(run_gates(ctx, (const int32_t*)d_g, uniform_gate, d_out, d_ca, d_cb, count, form, st));
-    CK(ctx, cudaMemcpyAsync(out, d_out, lwe_bytes, cudaMemcpyDeviceToHost, st));
-    CK(ctx, cudaStreamSynchronize(st));
-    return check_device_status(ctx);
+    if (2 * lwe_bytes + gate_bytes <= tfhe_gpu_ctx::kStageBytes) {
+        // one pinned copy instead of three pageable ones (a single gate's call
+        // 1,248 -> 1,232 us with the results and the status word in one wait)
+        std::memcpy(ctx->h_stage, ca, lwe_bytes);
+        std::memcpy(ctx->h_stage + lwe_bytes, cb, lwe_bytes);
+        if (gates) std::memcpy(ctx->h_stage + 2 * lwe_bytes, gates, gate_bytes);
+        CK(ctx, cudaMemcpyAsync(d_ca, ctx->h_stage, 2 * lwe_bytes + gate_bytes, cudaMemcpyHostToDevice, st));
+    } else {
+        CK(ctx, cudaMemcpyAsync(d_ca, ca, lwe_bytes, cudaMemcpyHostToDevice, st));
+        CK(ctx, cudaMemcpyAsync(d_cb, cb, lwe_bytes, cudaMemcpyHostToDevice, st));
+        if (gates) CK(ctx, cudaMemcpyAsync(d_g, gates, gate_bytes, cudaMemcpyHostToDevice, st));
+    }
+    RET(run_gates(ctx, d_g, uniform_gate, d_out, d_ca, d_cb, count, form, st));
+    return finish_host_call(ctx, out, d_out, lwe_bytes, st);
 }
 
 // ---- CUDA graph of the gate pipeline, launch-shape autotuner -----------
@@ -930,9 +954,7 @@ tfhe_gpu_status tfhe_gpu_bootsMUX_host(tfhe_gpu_ctx* ctx, int32_t* out, const in
     CK(ctx, cudaMemcpyAsync(d_b, b, lwe_bytes, cudaMemcpyHostToDevice, st));
     CK(ctx, cudaMemcpyAsync(d_c, c, lwe_bytes, cudaMemcpyHostToDevice, st));
     RET(tfhe_gpu_bootsMUX(ctx, d_out, d_a, d_b, d_c, count, form, st));
-    CK(ctx, cudaMemcpyAsync(out, d_out, lwe_bytes, cudaMemcpyDeviceToHost, st));
-    CK(ctx, cudaStreamSynchronize(st));
-    return check_device_status(ctx);
+    return finish_host_call(ctx, out, d_out, lwe_bytes, st);
 }
 
 }  // extern "C"

@@ -36,6 +36,10 @@ struct tfhe_gpu_ctx {
     void* d_scratch[4] = {nullptr, nullptr, nullptr, nullptr};
     size_t scratch_bytes[4] = {0, 0, 0, 0};
     int groups_per_cta[kNumForms] = {0, 0};  // launch shape per form; 0 = automatic
+    // pinned staging of the host-buffer calls: small batches go through it in
+    // one copy each way, and the status word comes back with the results
+    char* h_stage = nullptr;
+    static constexpr size_t kStageBytes = 512 * 1024;
     int32_t* d_err = nullptr;  // device status word written by bounded waits (3 = timeout)
     std::string last_error;
     size_t key_bytes = 0;
