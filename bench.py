@@ -13,13 +13,13 @@ seed 0, input bits from seed 4.  Synthetic data: no dataset is involved.
             (tfhe_gpu_bootsGates_host): pinned host ciphertexts in, results
             out, copies inside the timed region.
   roofline -- the dominant kernels (the blind-rotation launches of the
-            step, k_blind_rotate_ring for the 4096-gate layer) timed alone
-            with CUDA events: algorithmic FP work 162.6 MFLOP per bootstrap
+            step, k_blind_rotate_duo and k_blind_rotate_ring for the
+            4096-gate layer) timed alone with CUDA events: algorithmic FP work 162.6 MFLOP per bootstrap
             (FFT-form count) over their duration, against the FP32 FMA-pipe
             peak measured in the same run (tfhe_gpu_measure_fp32_peak).
-  roofline_smem -- the same kernels against the resource that bounds them:
-            shared-memory wavefronts per bootstrap (ncu counts of the same
-            kernels) over their duration, against one wavefront per SM clock.
+  roofline_smem -- the same kernels against the shared-memory pipe:
+            wavefronts per bootstrap (ncu counts of the same kernels) over
+            their duration, against one wavefront per SM clock.
   cpu_baseline -- the CPU oracle (restated reference path) on the host's
             cores on a bounded sample; beside it (fast_cpu) the same gates
             through a CPU bootstrap with the upstream library's N/2-point
@@ -57,12 +57,16 @@ FLOP_PER_BOOTSTRAP = 162.6e6      # FFT-form algorithmic count, default set
 # ciphertext moves 2.5 KB in and 4.5 KB out (66.5 MB measured for one
 # 608-gate wave of the batched ring kernel, 66.2 MB by this rule).
 DRAM_KEY_BYTES_PER_LAUNCH = 61.9e6
-# Shared-memory wavefronts per bootstrap of the two batched ring kernels
-# (the shared-memory wavefront count of a full ncu capture of each: 1.58 G
-# for a 912-gate wave, 0.74 G for a 448-gate wave; the capture is
-# summarised in profiles/blind_rotate_ring_pairs_batched_keyswitch_batch1360.md).
-# The shared-memory pipe serves one wavefront per SM clock.
+# Shared-memory wavefronts per bootstrap of the batched ring kernels (the
+# shared-memory wavefront count of a full ncu capture of each: 1.26 G for a
+# 912-gate wave in lane pairs, summarised in
+# profiles/kernels_lane_pairs_keyswitch_mma_fp64_cluster8.md; 0.74 G for a
+# 448-gate wave of the 4-per-SM kernel, and 1.58 G for the 6-per-SM kernel
+# before the lane pairs, both in
+# profiles/blind_rotate_ring_pairs_batched_keyswitch_batch1360.md).  The
+# shared-memory pipe serves one wavefront per SM clock.
 SMEM_WAVEFRONTS_PER_BOOTSTRAP = {
+    "k_blind_rotate_duo<3,3,4,2>": 1.26e9 / 912,
     "k_blind_rotate_ring<float,2,6,3,4,inline,nb2>": 1.58e9 / 912,
     "k_blind_rotate_ring<float,2,4,3,4,inline,nb3>": 0.74e9 / 448,
 }
@@ -919,7 +923,8 @@ def main():
         torch.cuda.synchronize()
         kms.append(e0.elapsed_time(e1))
     k_ms = statistics.median(kms)
-    br_launches = len(blind_rotate_kernels(args.form, eng.get_groups_per_cta(args.form), batch))
+    br_kernels = launched_blind_rotations(args.form, eng.get_groups_per_cta(args.form), batch)
+    br_launches = len(br_kernels)
     achieved = FLOP_PER_BOOTSTRAP * batch / (k_ms / 1000.0) / 1e12
     clocks = clk.summary()
     sm_max = clocks.get("sm_max_mhz") or 2070.0
@@ -1052,17 +1057,18 @@ def main():
             "decrypt_ok": ok,
             "e2e": {"value": e2e_value, "unit": "bootstraps/s",
                     "h2d_bytes_per_step": 2 * lwe_bytes + batch * 4, "d2h_bytes_per_step": lwe_bytes},
-            # eager: combine + per blind-rotation launch one key-switch launch
-            # (a split blind rotation has its key switch split the same way)
-            "gpu_launches": (graph.kernels if graph is not None else 1 + 2 * br_launches) * args.steps,
+            # eager: combine, the blind rotations, one key switch (two when full
+            # waves leave a remainder of at most 4 per SM)
+            "gpu_launches": (graph.kernels if graph is not None
+                             else 1 + br_launches + (2 if batch > 6 * SMS and 0 < batch % (6 * SMS) <= 4 * SMS else 1))
+            * args.steps,
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak,
                          "traffic": br_launches * DRAM_KEY_BYTES_PER_LAUNCH + batch * DRAM_IO_BYTES_PER_BOOTSTRAP,
                          "traffic_note": "DRAM bytes of the blind-rotation launches of one step, scaled from "
                                          "ncu captures of the same kernels (1360 gates): key once per "
                                          "launch + per-ciphertext I/O",
-                         "kernel": " + ".join(blind_rotate_kernels(args.form, eng.get_groups_per_cta(args.form),
-                                                                   batch)) + " (blind rotation + extraction)",
+                         "kernel": " + ".join(br_kernels) + " (blind rotation + extraction)",
                          "kernel_ms": k_ms,
                          "peak_source": "measured in this run: tfhe_gpu_measure_fp32_peak (independent packed "
                                         "FP32 FMA chains on every SM, CUDA events, %.1f ms; SM clock %s MHz); "
@@ -1070,8 +1076,7 @@ def main():
                                                                                      clk_peak.summary().get("sm_mhz")),
                          "nominal_peak": nominal_peak,
                          "frac_of_nominal": achieved / nominal_peak},
-            "roofline_smem": smem_roofline(blind_rotate_kernels(args.form, eng.get_groups_per_cta(args.form),
-                                                                batch), batch, k_ms, clocks),
+            "roofline_smem": smem_roofline(br_kernels, batch, k_ms, clocks),
             "clocks": clocks,
         }
         line.update(extras)
@@ -1154,9 +1159,53 @@ def smem_roofline(kernels, batch, k_ms, clocks):
             "note": "wavefronts per bootstrap from ncu counts of the same kernels, time from this run"}
 
 
+def launched_blind_rotations(form, shape, batch, l=3):
+    """Names of the blind-rotation kernels that a launch of `batch` runs with
+    launch shape `shape`: launch_auto_fp32, launch_auto_fp64 and the explicit
+    shapes of csrc/bootstrap.cu."""
+    duo = "k_blind_rotate_duo<%%d,%d,4,2>" % l
+    batched = duo % 2 if l == 2 else "k_blind_rotate_ring<float,2,4,%d,4,inline,nb%d>" % (l, l)
+
+    def low(cnt, pair=False):
+        tail = ",pair>" if pair else ">"
+        two, one = "k_blind_rotate_spread2<%d" % l + tail, "k_blind_rotate_spread<%d" % l + tail
+        if cnt <= SMS // 2:
+            return [two + " x %d" % cnt]
+        if SMS < cnt <= SMS + SMS // 2:
+            return [one + " x %d" % SMS, two + " x %d" % (cnt - SMS)]
+        return [one + " x %d" % cnt]
+
+    if form == "fp64" and shape == 0:
+        full = batch // (3 * SMS) * (3 * SMS)
+        if batch - full > 2 * SMS:
+            full = batch
+        rest = batch - full
+        names = ["k_external_product<double,1,BlindRotate,3,%d> x %d" % (l, full)] if full else []
+        if rest:
+            names += ["%s<%d> x %d" % ("k_blind_rotate_spread_f64" if rest > SMS // 2 else
+                                       "k_blind_rotate_cluster8_f64" if rest <= 48 else
+                                       "k_blind_rotate_spread2_f64", l, rest)]
+        return names
+    if form != "fp64" and shape in (0, 15):
+        full = batch // (6 * SMS) * (6 * SMS)
+        rest = batch - full
+        if rest == 0 or rest > 5 * SMS:
+            return [duo % 3 + " x %d" % batch]
+        names = [duo % 3 + " x %d" % full] if full else []
+        if rest > 2 * SMS:
+            most = min(rest, 4 * SMS)
+            names += [batched + " x %d" % most]
+            return names + (low(rest - most) if rest > most else [])
+        return names + low(rest, rest > SMS and shape == 0)
+    if form != "fp64" and shape in (9, 10):
+        return [batched if shape == 9 else duo % 3]
+    return blind_rotate_kernels(form, shape, batch, l)
+
+
 def blind_rotate_kernels(form, shape, batch, l=3):
-    """Names of the blind-rotation kernels a launch of `batch` runs with
-    launch shape `shape` (the engine's dispatch rules)."""
+    """Launch accounting by the shapes' first kernels: which shape a batch's
+    parts fall to, in those names (launched_blind_rotations has the kernels
+    that run them now)."""
     if form == "fp64":
         if shape == 16 or (shape == 0 and batch <= SMS):
             return ["k_blind_rotate_spread2_f64<%d>" % l]
