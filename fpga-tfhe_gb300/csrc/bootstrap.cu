@@ -1353,7 +1353,11 @@ struct SpreadPlan {
     static constexpr int kDB = L == 3 ? kHalf + 8 : 0;  // of level 2: [q][t], the next polynomial's 64 bytes round
     static constexpr int kD = kDA + kDB;
     static constexpr size_t acc_off = kHotSize * sizeof(cpx<float>);
-    static constexpr size_t d_off = acc_off + 2 * 2 * kN * sizeof(int32_t);  // two quadrants, see spread_put
+    // the accumulator's words, see spread_put: from one pair to the next, from
+    // one polynomial to the other
+    static constexpr int kAccPair = L == 2 ? 2 : 4;
+    static constexpr int kAccPoly = L == 2 ? 2 * kN : 2;
+    static constexpr size_t d_off = acc_off + 2 * 2 * kN * sizeof(int32_t);
     static constexpr size_t x_off = d_off + 2 * kD * sizeof(cpx<float>);
     static constexpr size_t key_off = x_off + kSets * kDuoSlots * sizeof(cpx<float>);
     static constexpr size_t bar_off = key_off + (size_t)kKeyParts * kKeyPart;  // 2 mbarriers, abort flag
@@ -1367,23 +1371,40 @@ struct SpreadPlan {
 // so that a rotation reads a folded point with one 64-bit load and needs only
 // a sign.  With A and B the coefficients u and u + 512 (u < 512), s = u holds
 // (A, B) and s = u + 512 holds (B, -A).
+//
+// For l = 2 every set reads one polynomial, whose pairs lie one after the
+// other: the 16 points that a warp's lane pairs read, or write as 32 words, are
+// one wavefront.  With the pairs of both polynomials side by side they are
+// two (256 wavefronts of a step more): 1.079 -> 1.000 ms for 152 ciphertexts,
+// 2.078 -> 2.033 ms for 304.  For l = 3, whose third set reads both polynomials
+// at once, the side by side form is the faster one although it has those
+// wavefronts: 1.574 against 1.598 ms for 152 ciphertexts, 3.05 against 3.20 ms
+// for 304.  (The addresses are written out per form: one expression for both
+// cost l = 2 0.028 ms, and l = 3 0.02 ms the other way round.)
+template <int L>
 __device__ __forceinline__ int spread_word(int j, int x) {  // of coefficient x < N
-    return ((x & (kHalf - 1)) * 2 + j) * 2 + (x >> 9);
+    return L == 2 ? j * SpreadPlan<L>::kAccPoly + (x & (kHalf - 1)) * SpreadPlan<L>::kAccPair + (x >> 9)
+                  : ((x & (kHalf - 1)) * 2 + j) * 2 + (x >> 9);
 }
+template <int L>
 __device__ __forceinline__ void spread_put(int32_t* acc, int j, int x, uint32_t v) {
     const int half = x >> 9;
-    int32_t* w = acc + ((x & (kHalf - 1)) * 2 + j) * 2;
+    int32_t* w = L == 2 ? acc + j * SpreadPlan<L>::kAccPoly + (x & (kHalf - 1)) * SpreadPlan<L>::kAccPair
+                        : acc + ((x & (kHalf - 1)) * 2 + j) * 2;
     w[half] = (int32_t)v;
-    w[kHalf * 4 + 1 - half] = (int32_t)(half ? v : 0u - v);
+    w[kHalf * SpreadPlan<L>::kAccPair + 1 - half] = (int32_t)(half ? v : 0u - v);
 }
 // X^a - 1 applied to the folded point t + 64r of polynomial j, plus the
 // gadget offset: r0 for coefficient t + 64r, r1 for that + 512.
+template <int L>
 __device__ __forceinline__ void rotated_pair(const int32_t* acc, int j, int t, int r, int a, uint32_t offset,
                                              uint32_t& r0, uint32_t& r1) {
-    const int2* src = reinterpret_cast<const int2*>(acc) + j;
+    constexpr int kStep = SpreadPlan<L>::kAccPair / 2;
+    const int2* src = L == 2 ? reinterpret_cast<const int2*>(acc + j * SpreadPlan<L>::kAccPoly)
+                             : reinterpret_cast<const int2*>(acc) + j;
     const int s = t + 64 * r - a;
-    const int2 w = src[(s & (kN - 1)) * 2];
-    const int2 p = src[(t + 64 * r) * 2];
+    const int2 w = src[(s & (kN - 1)) * kStep];
+    const int2 p = src[(t + 64 * r) * kStep];
     const uint32_t m = (uint32_t)((s << 21) >> 31);  // all ones when s mod 2N >= N
     r0 = ((uint32_t)w.x ^ m) - (uint32_t)p.x + (offset - m);
     r1 = ((uint32_t)w.y ^ m) - (uint32_t)p.y + (offset - m);
@@ -1411,13 +1432,13 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
     if (a.acc_in) {
         const int32_t* src = a.acc_in + (size_t)c * 2 * kN;
         for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x)
-            spread_put(acc, i >> 10, i & (kN - 1), (uint32_t)src[i]);
+            spread_put<L>(acc, i >> 10, i & (kN - 1), (uint32_t)src[i]);
     } else {
         const int32_t* xs = a.x + (size_t)c * (n + 1);
         const int barb = mod_switch_2n(xs[n]);
         for (int i = threadIdx.x; i < kN; i += blockDim.x) {
-            spread_put(acc, 0, i, 0u);
-            spread_put(acc, 1, i, (uint32_t)test_vector_coef(a, c, barb, i));
+            spread_put<L>(acc, 0, i, 0u);
+            spread_put<L>(acc, 1, i, (uint32_t)test_vector_coef(a, c, barb, i));
         }
     }
     if (threadIdx.x == 0) {
@@ -1475,7 +1496,7 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
         uint32_t own[8] = {};  // owners: coefficients t + 64q (even lane) or 512 above (odd) of the output polynomial
         if (owner) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) own[q] = (uint32_t)acc[spread_word(set, t + 64 * q + e * kHalf)];
+            for (int q = 0; q < 8; ++q) own[q] = (uint32_t)acc[spread_word<L>(set, t + 64 * q + e * kHalf)];
         }
         const int32_t* bara = a.bara ? a.bara + (size_t)c * n : nullptr;
         const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
@@ -1497,7 +1518,7 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 uint32_t u0, u1;
-                rotated_pair(acc, jp, t, q, ai, kp.offset, u0, u1);
+                rotated_pair<L>(acc, jp, t, q, ai, kp.offset, u0, u1);
                 v[0][q] = digit_pair<float>(u0, u1, decal, mask, halfBg);
             }
             fft512_forward_duo<1>(v, xbuf, tw, ix, bar_id);
@@ -1557,7 +1578,7 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
                     c1 <<= out_shift;
                     const uint32_t other = __shfl_xor_sync(0xffffffffu, e ? c0 : c1, 1);
                     own[q] += (e ? c1 : c0) + other;
-                    spread_put(acc, set, t + 64 * q + e * kHalf, own[q]);
+                    spread_put<L>(acc, set, t + 64 * q + e * kHalf, own[q]);
                 }
             }
             step_sync();  // the accumulator is updated before the next step reads it
@@ -1566,14 +1587,14 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
     __syncthreads();
     if (a.acc_out) {
         int32_t* dst = a.acc_out + (size_t)c * 2 * kN;
-        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x) dst[i] = acc[spread_word(i >> 10, i & (kN - 1))];
+        for (int i = threadIdx.x; i < 2 * kN; i += blockDim.x) dst[i] = acc[spread_word<L>(i >> 10, i & (kN - 1))];
     }
     if (a.lwe_out) {
         // tLweExtractLweSample: a'_0 = a_0, a'_j = -a_{N-j}, b' = b_0
         int32_t* dst = a.lwe_out + (size_t)c * (kN + 1);
         for (int i = threadIdx.x; i < kN; i += blockDim.x)
-            dst[i] = i == 0 ? acc[spread_word(0, 0)] : (int32_t)(0u - (uint32_t)acc[spread_word(0, kN - i)]);
-        if (threadIdx.x == 0) dst[kN] = acc[spread_word(1, 0)];
+            dst[i] = i == 0 ? acc[spread_word<L>(0, 0)] : (int32_t)(0u - (uint32_t)acc[spread_word<L>(0, kN - i)]);
+        if (threadIdx.x == 0) dst[kN] = acc[spread_word<L>(1, 0)];
     }
 }
 
