@@ -67,6 +67,7 @@ DRAM_KEY_BYTES_PER_LAUNCH = 61.9e6
 # shared-memory pipe serves one wavefront per SM clock.
 SMEM_WAVEFRONTS_PER_BOOTSTRAP = {
     "k_blind_rotate_duo<3,3,4,2>": 1.26e9 / 912,
+    "k_blind_rotate_ring<float,2,3,3,4,inline,nb3>": 0.74e9 / 448,
     "k_blind_rotate_ring<float,2,6,3,4,inline,nb2>": 1.58e9 / 912,
     "k_blind_rotate_ring<float,2,4,3,4,inline,nb3>": 0.74e9 / 448,
 }
@@ -1164,7 +1165,11 @@ def launched_blind_rotations(form, shape, batch, l=3):
     launch shape `shape`: launch_auto_fp32, launch_auto_fp64 and the explicit
     shapes of csrc/bootstrap.cu."""
     duo = "k_blind_rotate_duo<%%d,%d,4,2>" % l
-    batched = duo % 2 if l == 2 else "k_blind_rotate_ring<float,2,4,%d,4,inline,nb%d>" % (l, l)
+
+    def batched(cnt):
+        if cnt > 3 * SMS and l == 2:
+            return duo % 2
+        return "k_blind_rotate_ring<float,2,%d,%d,4,inline,nb%d>" % (4 if cnt > 3 * SMS else 3, l, l)
 
     def low(cnt, pair=False):
         tail = ",pair>" if pair else ">"
@@ -1194,11 +1199,11 @@ def launched_blind_rotations(form, shape, batch, l=3):
         names = [duo % 3 + " x %d" % full] if full else []
         if rest > 2 * SMS:
             most = min(rest, 4 * SMS)
-            names += [batched + " x %d" % most]
+            names += [batched(most) + " x %d" % most]
             return names + (low(rest - most) if rest > most else [])
         return names + low(rest, rest > SMS and shape == 0)
     if form != "fp64" and shape in (9, 10):
-        return [batched if shape == 9 else duo % 3]
+        return [batched(batch) if shape == 9 else duo % 3]
     return blind_rotate_kernels(form, shape, batch, l)
 
 

@@ -513,9 +513,9 @@ class Engine:
         """Launch shape of the blind rotation (tfhe_gpu_set_groups_per_cta).
         split_fp32: 0 automatic; 1, 2, 4 L2-direct; 5-8 shared key ring, one
         transform at a time; 9 ring, 4 per CTA, a step's transforms
-        together; 10 ring, 6 per CTA, two at a time; 11-13 pair kernel;
-        14 spread kernel; 15 automatic in fixed summation order (no pair
-        kernel: results independent of the batch); 16 spread kernel over a
+        together; 10 ring, 6 per CTA in lane pairs; 11-13 pair kernel;
+        14 spread kernel; 15 automatic in fixed summation order (never the
+        pair kernel's: results independent of the batch); 16 spread kernel over a
         two-SM cluster (lowest latency).  fp64: 0 automatic (waves of 3 per SM
         on shape 3, smaller remainders on the one-per-CTA, the two-SM or
         the eight-SM cluster kernel); 3 L2-direct, 3 per CTA; 4 shared key ring; 16 two-SM cluster."""

@@ -1337,7 +1337,7 @@ __global__ void __launch_bounds__(kDuoThreads * SETS, 1) k_blind_rotate_duo(KPar
 // Measured against the form with one transform per 64 threads, the high and
 // the low part in different groups, keys loaded into registers (the loads
 // held the load/store unit for 600 clocks a step) and accumulated by
-// shared-memory atomics: 1.755 -> 1.587 ms for 152 ciphertexts; the twiddles
+// shared-memory atomics: 1.755 -> 1.574 ms for 152 ciphertexts; the twiddles
 // in registers instead of shared memory are 0.054 ms of that.
 // ----------------------------------------------------------------------
 template <int L>
@@ -3064,9 +3064,13 @@ cudaError_t launch_duo(const DevParams& P, const Tables& T, const EpArgs& a, cud
 // three forward transforms run together in one ciphertext's 64 threads (4.56
 // ms for 608; in lane pairs two at a time 4.71 ms), for l = 2 in lane pairs
 // (2.79 ms against 2.90) -- or 6 per CTA in lane pairs, transforms two at a
-// time (168 registers, 12 warps per SM).
+// time (168 registers, 12 warps per SM).  What 3 per SM can hold runs as 3
+// per CTA with a step's transforms together, on more SMs with fewer warps
+// each: 448 ciphertexts 4.54 -> 4.29 ms, 305 4.49 -> 4.17 ms, l = 2 448 2.78
+// -> 2.68 ms.
 template <int L>
 cudaError_t launch_ring_batched(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
+    if (a.count <= 3 * kSmCount) return launch_ring_t<float, 2, 3, L, true, 4, L>(P, T, a, st);
     if constexpr (L == 2) return launch_duo<2, L>(P, T, a, st);
     else return launch_ring_t<float, 2, 4, L, true, 4, L>(P, T, a, st);
 }
@@ -3090,8 +3094,8 @@ cudaError_t launch_low_latency(const DevParams& P, const Tables& T, const EpArgs
 
 // Automatic shape of a split-FP32 blind rotation over `count` ciphertexts.
 // Measured per launch (default set): a wave of 6 per SM on
-// launch_ring_pairs 6.2 ms, of 4 per SM on launch_ring_batched 4.6 ms,
-// whatever the fill of the wave; the cluster kernel 1.12 ms for up to one
+// launch_ring_pairs 6.2 ms, of 4 per SM on launch_ring_batched 4.6 ms (4.2
+// to 4.3 ms up to 3 per SM), whatever the fill of the wave; the cluster kernel 1.12 ms for up to one
 // per two SMs; the spread kernel 1.58 ms at 1 per SM, 3.0 to 3.2 ms for two
 // waves.  So: whole waves of 6 per SM; a remainder of up to 2 per SM on those
 // two (2.7 ms up to 1.5 per SM, where the pair kernel took 3.24 ms for any

@@ -103,24 +103,28 @@ size_t tfhe_gpu_device_bytes(const tfhe_gpu_ctx* ctx);
 /* Launch shape of the blind-rotation kernel of `form`.  split-FP32:
  *   0 = automatic: whole waves of 6 ciphertexts per SM on shape 10; a
  *       remainder of at most one per two SMs on shape 16, of at most 1 per
- *       SM on shape 14, of 2 per SM on the pair kernel, of at most 4 per SM
- *       as one shape-9 wave, else one more shape-10 wave;
+ *       SM on shape 14, of at most 2 per SM on these two in the pair kernel's
+ *       summation order, of at most 4 per SM as one shape-9 wave, of at most
+ *       5 per SM as a full shape-9 wave and the rest by the rules before,
+ *       else one more shape-10 wave;
  *   1, 2, 4 = ciphertexts (64 threads each) per CTA, key rows read from L2
  *       by every ciphertext;
  *   5 = 5 per CTA, key rows streamed once per CTA into a shared-memory ring
  *       by a producer warp;
  *   6, 7, 8 = that many per CTA, the same ring fed by one consumer thread;
- *   9 = 4 per CTA on the same ring, each step's l forward and 2 inverse
- *       transforms run together (about 250 registers a thread);
- *   10 = 6 per CTA on the same ring, transforms two at a time;
+ *   9 = 4 per CTA on the same ring, each step's 3 forward and 2 inverse
+ *       transforms run together (about 250 registers a thread; l = 2: as
+ *       10); 3 per CTA for launches of at most 3 per SM;
+ *   10 = 6 per CTA on the same ring, two ciphertexts in the lane pairs of 128
+ *       threads, transforms two at a time;
  *   11, 12, 13 = pair kernel: two 64-thread halves per ciphertext (about
  *       half the latency), 1, 2, 3 ciphertexts per CTA, shared ring;
  *   14 = spread kernel: one ciphertext per CTA over l sets of 128 threads,
  *       two transforms each; two of the sets multiply all rows for one output
  *       polynomial and transform it back (low latency up to one per SM), key
  *       rows copied ahead by a producer warp;
- *   15 = automatic in fixed summation order: as 0, with the spread kernel
- *       (two waves) in place of the pair kernel, whose two halves' partial
+ *   15 = automatic in fixed summation order: as 0, without the pair
+ *       kernel's order for 1 to 2 per SM, whose two halves' partial
  *       products round differently; every launch then sums the key rows in
  *       the same order, and a ciphertext's result is the same bit for bit
  *       whatever batch it runs in (the gate server uses it);

@@ -113,6 +113,23 @@ def test_lane_pair_ring_matches_l2_direct(engines, torch_cuda, params, shape, co
                 == _rotations(torch, e, "split_fp32", 4, acc, bara)).all()
 
 
+# shape 9 as 3 per CTA up to 3 per SM: a part of a CTA, the last count of it, one more
+@pytest.mark.parametrize("params,shape,count", [("default", 9, 2), ("default", 0, 305), ("stress", 0, 456), ("stress", 9, 457),
+                                                ("default", 0, 912 + 457)])
+def test_three_per_sm_ring_matches_l2_direct(engines, torch_cuda, params, shape, count):
+    torch = torch_cuda
+    e = engines(params)
+    x = _uniform(torch, count, count, e.params.n + 1)
+    x[0, 7] = 0
+    assert (_bootstraps(torch, e, "split_fp32", shape, x) == _bootstraps(torch, e, "split_fp32", 4, x)).all()
+    if count < 10:
+        acc = _uniform(torch, 3, count, 2048)
+        bara = _uniform(torch, 4, count, e.params.n) & 2047
+        bara[:, 5] = 0
+        assert (_rotations(torch, e, "split_fp32", shape, acc, bara)
+                == _rotations(torch, e, "split_fp32", 4, acc, bara)).all()
+
+
 # shape 0 over 1 to 2 per SM keeps the pair kernel's summation order (shape 12)
 # whatever runs it; shape 15, and shape 0 elsewhere, the order of the rows
 # (shape 4): edges of 1, 1.5, 2, 4, 4.5 and 5 per SM, and after a full wave
