@@ -1697,6 +1697,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
     // side jobs of the last warp, done once its group's digits are out: with
     // l = 3 that group owns no output (they cost a warp 230 clocks a step)
     const int side = (int)threadIdx.x - (64 * L - 32);
+    // Key rows go into L2 eight steps (14 us) ahead.  A gate's key switch
+    // streams its table between two blind rotations, so the bootstrapping key
+    // comes from HBM again: after a key switch 1,179 -> 1,170 us for one
+    // ciphertext and 1,160 -> 1,153 us for 64 against two steps ahead (four:
+    // no gain; sixteen: slower).
+    constexpr int kAhead = 8;
     const auto prefetch_rows = [&](int step) {
         if (step < n && side >= 0 && side < kRows && (side & 1) == r)
             bulk_prefetch_l2(gsw + (size_t)step * step_elems + (size_t)side * kRowElems,
@@ -1706,8 +1712,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
     const auto expect_digits = [&](int b) {
         if (side == 0) mbar_arrive_expect_tx(&dbar[b], (uint32_t)(L * kHalf * sizeof(cpx<float>)));
     };
-    prefetch_rows(0);
-    prefetch_rows(1);
+    for (int s = 0; s < kAhead; ++s) prefetch_rows(s);
     expect_digits(0);
     uint32_t k = 0;  // steps taken (the same in both CTAs)
 #pragma unroll 1
@@ -1749,7 +1754,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
             }
         }
         __syncthreads();  // every local D in place; every read of acc done
-        prefetch_rows(i + 2);
+        prefetch_rows(i + kAhead);
         expect_digits(buf ^ 1);  // the other buffer's last digits were used a step ago
         if (owner) {
             if (!mbar_wait_cluster_bounded(&dbar[buf], (k >> 1) & 1, abort)) {  // the peer's D landed
