@@ -29,6 +29,7 @@
 #include "async_copy.cuh"
 #include "engine.h"
 #include "fft512.cuh"
+#include "key_stream.cuh"
 
 namespace tfhe_gb300 {
 
@@ -650,54 +651,14 @@ __global__ void __launch_bounds__(64 * GROUPS, 1) k_external_product(KParams kp,
 template <int L>
 struct ProductPlan {
     static constexpr int kGroups = 4;
-    static constexpr int S = 2;  // row slots per group
-    static constexpr size_t kRowBytes = (size_t)2 * 2 * kHalf * sizeof(cpx<float>);
+    static constexpr int S = ItemKeys<L>::S;
+    static constexpr size_t kRowBytes = ItemKeys<L>::kRowBytes;
     static constexpr size_t ring_off = (kHotSize * sizeof(cpx<float>) + 127) & ~(size_t)127;
     static constexpr size_t x_off = ring_off + kGroups * S * kRowBytes;
     static constexpr size_t x_group = 4 * kScratchStride * sizeof(cpx<float>);  // two transforms, two buffers each
     static constexpr size_t bar_off = x_off + kGroups * x_group;
     static constexpr size_t flag_off = bar_off + kGroups * S * sizeof(uint64_t);
     static constexpr size_t total = flag_off + 16;
-};
-
-// This group's row stream: row r is row r % 2l of the group's item r / 2l.
-template <int L>
-struct ItemKeys {
-    static constexpr int S = ProductPlan<L>::S;
-    static constexpr size_t kRowBytes = ProductPlan<L>::kRowBytes;
-    cpx<float>* ring;
-    uint64_t* full;
-    int32_t* err;
-    volatile int* abort;
-    const char* src;     // first item
-    size_t item_stride;  // bytes from one item of the group to the next
-    uint32_t total, next, used;
-    int t;
-
-    // thread 0: rows up to used + S - 1 (all earlier uses of their slots are over)
-    __device__ __forceinline__ void issue() {
-        for (; next < total && next < used + S; ++next) {
-            const uint32_t slot = next % S, item = next / (2 * L), row = next - item * (2 * L);
-            mbar_arrive_expect_tx(&full[slot], (uint32_t)kRowBytes);
-            bulk_copy_g2s(reinterpret_cast<char*>(ring) + slot * kRowBytes,
-                          src + item * item_stride + row * kRowBytes, (uint32_t)kRowBytes, &full[slot]);
-        }
-    }
-    __device__ __forceinline__ const cpx<float>* wait(uint32_t r) {
-        if (!mbar_wait_bounded(&full[r % S], (r / S) & 1, abort)) {
-            *abort = 1;
-            atomicExch(err, 3);
-        }
-        __syncwarp();
-        return ring + (r % S) * (kRowBytes / sizeof(cpx<float>));
-    }
-    // the group is done with its next `rows` rows
-    __device__ __forceinline__ void release(int rows, int bar_id) {
-        used += rows;
-        group_sync(bar_id);
-        if (t == 0) issue();
-        __syncwarp();
-    }
 };
 
 template <int NBK, int L>
@@ -813,6 +774,7 @@ __global__ void __launch_bounds__(64 * ProductPlan<L>::kGroups, 1)
         }
         group_sync(bar_id);  // the exchange buffers are free for the next item
     }
+    if (t == 0) keys.drain();
 }
 
 // ----------------------------------------------------------------------

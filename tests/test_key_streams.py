@@ -1,0 +1,32 @@
+"""The key-row streams (csrc/key_stream.cuh) on a host model of the barriers,
+with one row's copy that never lands (or none): the stream ends by itself,
+arms no slot whose copy is out, and waits for what it has issued.  CPU only."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "fpga-tfhe_gb300", "csrc")
+
+
+@pytest.fixture(scope="module")
+def model(tmp_path_factory):
+    if not shutil.which("g++"):
+        pytest.skip("no g++")
+    exe = str(tmp_path_factory.mktemp("streams") / "key_streams")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, "-o", exe, os.path.join(HERE, "key_streams.cpp")],
+                   check=True, capture_output=True)
+
+    def run(what, lost):
+        return subprocess.run([exe, what, str(lost)], capture_output=True, text=True).stdout.split("\n")[:-1]
+
+    return run
+
+
+# no row lost; the first, one whose slot has a next use, the last two
+@pytest.mark.parametrize("stream,rows", [("products2", 12), ("products3", 18)])
+def test_product_stream_ends_by_itself(model, stream, rows):
+    for lost in (-1, 0, 3, 6, rows - 2, rows - 1):
+        assert model(stream, lost) == [], lost
