@@ -171,6 +171,7 @@ SIGNATURES = {
     "tfhe_client_test_vector": (ctypes.c_int, [ctypes.c_int32, I32P, ctypes.c_int32, I32P]),
     "tfhe_gpu_gate_keyset": (ctypes.c_int, [VP, I32P, I32P, I32P, I32P, ctypes.c_uint32]),
     "tfhe_gpu_selftest_timeout": (ctypes.c_int, [VP, ctypes.c_int, ctypes.c_int32]),
+    "tfhe_gpu_selftest_timeout_in": (ctypes.c_int, [VP, ctypes.c_int32, ctypes.c_int32]),
     "tfhe_gpu_measure_fp32_peak": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32,
                                                   ctypes.POINTER(ctypes.c_double),
                                                   ctypes.POINTER(ctypes.c_double)]),
@@ -565,6 +566,10 @@ class Engine:
         bounded waits run out): 3 = TFHE_GPU_TIMEOUT, 0 for shapes without
         waits."""
         return self.lib.tfhe_gpu_selftest_timeout(self.ctx, self._form(form), int(count))
+
+    def selftest_timeout_in(self, part, count):
+        """The same for another part of the engine: "key_switch"."""
+        return self.lib.tfhe_gpu_selftest_timeout_in(self.ctx, {"key_switch": 1}[part], int(count))
 
     def autotune(self, form, count):
         """Time the launch shapes on `count` ciphertexts; keeps and returns

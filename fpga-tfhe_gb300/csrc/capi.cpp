@@ -935,6 +935,24 @@ tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form,
     return check_device_status(ctx);
 }
 
+tfhe_gpu_status tfhe_gpu_selftest_timeout_in(tfhe_gpu_ctx* ctx, int32_t part, int32_t count) {
+    CHECK_CTX(ctx);
+    if (count <= 0 || part != TFHE_GPU_PART_KEY_SWITCH) return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
+    RET(check_device_status(ctx));  // start from a clean status word
+    const int n = ctx->P.n, nk = ctx->P.k * ctx->P.N;
+    cudaStream_t st = ctx->stream;
+    void *u = nullptr, *out = nullptr;
+    if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
+    RET(ensure_scratch(ctx, 1, (size_t)count * (nk + 1) * sizeof(int32_t), &u));
+    RET(ensure_scratch(ctx, 0, (size_t)count * (n + 1) * sizeof(int32_t), &out));
+    CK(ctx, cudaMemsetAsync(u, 0, (size_t)count * (nk + 1) * sizeof(int32_t), st));
+    KsTable ks = ctx->ks_table();
+    ks.stall = true;
+    CK(ctx, launch_keyswitch(ctx->dp, ks, (const int32_t*)u, (int32_t*)out, count, st));
+    CK(ctx, cudaStreamSynchronize(st));
+    return check_device_status(ctx);
+}
+
 tfhe_gpu_status tfhe_gpu_bootsMUX_host(tfhe_gpu_ctx* ctx, int32_t* out, const int32_t* a,
                                        const int32_t* b, const int32_t* c, int32_t count,
                                        tfhe_gpu_form form) {

@@ -31,7 +31,7 @@ struct tfhe_gpu_ctx {
     int32_t* d_ks = nullptr;
     bool has_ks() const { return d_ks || d_ks_tiles; }
     int32_t ks_row_stride = 0;
-    tfhe_gb300::KsTable ks_table() const { return {d_ks, ks_row_stride, d_ks_tiles, d_err}; }
+    tfhe_gb300::KsTable ks_table() const { return {d_ks, ks_row_stride, d_ks_tiles, d_err, false}; }
     // scratch slots, grown on demand
     void* d_scratch[4] = {nullptr, nullptr, nullptr, nullptr};
     size_t scratch_bytes[4] = {0, 0, 0, 0};

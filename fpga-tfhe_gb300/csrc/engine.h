@@ -123,12 +123,14 @@ int blind_rotate_tail_start(Form f, int groups, int count);
 // Key-switching table on the device: for t = 8 its words in FP16 pieces in
 // the tensor cores' order (tiles), for other t rows `row_stride` int32 apart,
 // layout [kN][t][base][row_stride]; the other pointer is null.  err: device
-// status word.
+// status word.  stall: self-test of the bounded waits, the table's stream ends
+// after its first stage (tfhe_gpu_selftest_timeout_in).
 struct KsTable {
     const int32_t* rows;
     int32_t row_stride;
     const void* tiles;
     int32_t* err;
+    bool stall;
 };
 // Key switching: in (count x (kN+1)) -> out (count x (n+1)).
 cudaError_t launch_keyswitch(const DevParams& P, const KsTable& ks, const int32_t* in,
@@ -139,7 +141,7 @@ size_t keyswitch_tile_bytes(const DevParams& P);
 cudaError_t launch_keyswitch_tiles(const DevParams& P, const int32_t* ks, int32_t row_stride,
                                    void* tiles, cudaStream_t st);
 cudaError_t launch_keyswitch_mma(const DevParams& P, const void* tiles, const int32_t* in, int32_t* out,
-                                 int count, int32_t* err, cudaStream_t st);
+                                 int count, int32_t* err, cudaStream_t st, bool stall);
 
 // Finish n TGSW encryptions whose rows hold masks a and noise b = e (host
 // RNG, exact order): b += sum_i a_i * s_i (negacyclic, TLWE key s, N k

@@ -138,7 +138,7 @@ cudaError_t launch_keyswitch(const DevParams& P, const KsTable& table, const int
     // t = 8 runs on the tensor cores whatever the count (4,096 key switches
     // 2.88 -> 0.246 ms, 64 0.087 -> 0.031 ms, one 29 -> 27 us); this kernel
     // serves t = 4 and 12
-    if (table.tiles) return launch_keyswitch_mma(P, table.tiles, in, out, count, table.err, st);
+    if (table.tiles) return launch_keyswitch_mma(P, table.tiles, in, out, count, table.err, st, table.stall);
     const int32_t* ks = table.rows;
     const int row_stride = table.row_stride;
     if (P.ks_basebit != 2 || P.ks_t % kKsJBlock || P.ks_t > 16 || (row_stride & 3) ||

@@ -103,7 +103,7 @@ __device__ __forceinline__ uint4 one_hot(uint32_t u, uint32_t h) {
 
 __global__ void __launch_bounds__(kThreads, 1)
     k_keyswitch_mma(const void* __restrict__ tiles, const int32_t* __restrict__ in, int32_t* __restrict__ out, int count,
-                    int n, int n_in, int parts, int32_t* err) {
+                    int n, int n_in, int parts, int32_t* err, int stall) {
     extern __shared__ __align__(128) char smem[];
     uint64_t* full_a = reinterpret_cast<uint64_t*>(smem + kBarOff);
     uint64_t* full_b = full_a + kStages;
@@ -187,13 +187,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if ((threadIdx.x & 31) == 0) mbar_arrive(&full_a[q]);
             }
         }
-        if (!mbar_wait_bounded(done, 0, abort)) gave_up();
-        __syncwarp();
+        // without the abort flag: `done` completes after the last matrix
+        // instruction that was issued, also when a wait has given up
+        bool summed = mbar_wait_bounded(done, 0);
+        if (!summed) gave_up();
+        summed = __all_sync(0xffffffffu, summed);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // row 32 (warp % 4) + lane of half warp / 4, 16 output words at a time
         const int half = warp >> 2;
         const uint32_t taddr = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)half * 256;
-        if (half == 0 || two) {
+        if (summed && (half == 0 || two)) {
             const int col0 = tile * kTileC;
             const uint32_t body = live && part == 0 ? (uint32_t)in[(size_t)c * (n_in + 1) + n_in] : 0u;
             int32_t* o = out + (size_t)(live ? c : c0) * (n + 1) + col0;
@@ -240,6 +243,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 mma_commit(&empty[q]);
             }
             mma_commit(done);
+            // the accumulators are freed below, with no matrix instruction in flight
+            if (!mbar_wait_bounded(done, 0)) atomicExch(err, 3);
         }
         __syncwarp();
     } else {
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                               ((size_t)tile * n_in + (size_t)s0 * kStageCoefs) * (3 * kBChunk);
             int issued = 0;
 #pragma unroll 1
-            for (int it = 0; it < stages; ++it, ++issued) {
+            for (int it = 0; it < (stall ? min(stages, 1) : stages); ++it, ++issued) {
                 const int q = it % kStages;
                 if (it >= kStages && !mbar_wait_bounded(&empty[q], ((it / kStages) - 1) & 1, abort)) {
                     gave_up();
@@ -323,7 +328,7 @@ cudaError_t launch_keyswitch_tiles(const DevParams& P, const int32_t* ks, int32_
 }
 
 cudaError_t launch_keyswitch_mma(const DevParams& P, const void* tiles, const int32_t* in, int32_t* out, int count,
-                                 int32_t* err, cudaStream_t st) {
+                                 int32_t* err, cudaStream_t st, bool stall) {
     if (count <= 0) return cudaSuccess;
     const int n_in = P.k * P.N;
     const int blocks = ((count + kTileM - 1) / kTileM) * ((P.n + kTileC) / kTileC);
@@ -337,7 +342,7 @@ cudaError_t launch_keyswitch_mma(const DevParams& P, const void* tiles, const in
         e = cudaMemsetAsync(out, 0, (size_t)count * (P.n + 1) * sizeof(int32_t), st);
         if (e != cudaSuccess) return e;
     }
-    k_keyswitch_mma<<<blocks * parts, kThreads, kSmem, st>>>(tiles, in, out, count, P.n, n_in, parts, err);
+    k_keyswitch_mma<<<blocks * parts, kThreads, kSmem, st>>>(tiles, in, out, count, P.n, n_in, parts, err, stall);
     return cudaGetLastError();
 }
 

@@ -332,6 +332,11 @@ tfhe_gpu_status tfhe_gpu_bootsGates_noalloc(tfhe_gpu_ctx* ctx, const int32_t* ga
  * shared-ring shapes; TFHE_GPU_OK for the L2-direct shapes, which have no
  * waits.  The context stays usable.  No counterpart in the reference. */
 tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form, int32_t count);
+/* The same for another part of the engine, over `count` samples:
+ *   TFHE_GPU_PART_KEY_SWITCH: a key switch whose table stream ends after its
+ *     first stage (TFHE_GPU_OK for ks_t other than 8, which has no waits). */
+#define TFHE_GPU_PART_KEY_SWITCH 1
+tfhe_gpu_status tfhe_gpu_selftest_timeout_in(tfhe_gpu_ctx* ctx, int32_t part, int32_t count);
 
 /* Measured FP32 FMA-pipe peak of `device` in TFLOP/s (and the probe's
  * duration in ms): independent chains of packed FP32 fused multiply-adds on

@@ -1,0 +1,44 @@
+"""Bounded waits that run out, part by part: the call ends within a few seconds
+with TFHE_GPU_TIMEOUT, and the same context then works.  The waits run out
+because a stream is not fed (a flag of the self-test), not by a fault."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _timeout_then(run, check):
+    t0 = time.perf_counter()
+    st = run()
+    assert st == 3, st
+    assert time.perf_counter() - t0 < 30
+    check()
+
+
+# one tile with few stages a CTA, both halves of a tile, whole coefficient range in a CTA
+@pytest.mark.parametrize("count", [1, 200, 8000])
+def test_key_switch_timeout(pkg, torch_cuda, count):
+    torch = torch_cuda
+    P = pkg.default_params()
+    e = pkg.Engine(P)
+    try:
+        ks = np.random.default_rng(3).integers(-2 ** 31, 2 ** 31, P.ks_words()).astype(np.int32)
+        e.upload_keyswitch_key(ks)
+        x = torch.randint(-2 ** 31, 2 ** 31, (count, 1025), device="cuda", dtype=torch.int32)
+        out = torch.empty((2, count, P.n + 1), device="cuda", dtype=torch.int32)
+        sp = torch.cuda.current_stream().cuda_stream
+        e.lweKeySwitch(out[0], x, count, stream=sp)
+        torch.cuda.synchronize()
+
+        def check():
+            e.synchronize()
+            e.lweKeySwitch(out[1], x, count, stream=sp)
+            torch.cuda.synchronize()
+            e.synchronize()
+            assert torch.equal(out[0], out[1])
+
+        _timeout_then(lambda: e.selftest_timeout_in("key_switch", count), check)
+    finally:
+        e.close()
