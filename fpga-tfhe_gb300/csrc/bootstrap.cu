@@ -788,128 +788,10 @@ __global__ void __launch_bounds__(64 * ProductPlan<L>::kGroups, 1)
 // L2 latency on the multiply-accumulate.  Slot hand-off uses two mbarriers
 // per slot: full (the copy's byte count landed) and empty (every consumer
 // thread has read the row).  A group that skips a step (a_i = 0) still waits
-// and releases its rows, so the ring stays in step.  Every wait is bounded;
-// a timeout sets *err (TFHE_GPU_TIMEOUT for the host) and the kernel runs to
-// its end without further waiting on the ring.
+// and releases its rows, so the ring stays in step (RingKeys).  Every wait is
+// bounded; a timeout sets *err (TFHE_GPU_TIMEOUT for the host) and the kernel
+// runs to its end without further waiting on the ring.
 // ----------------------------------------------------------------------
-template <typename R, int PARTS, int S>
-struct RingKeys {
-    static constexpr size_t kRow = (size_t)2 * PARTS * kHalf;
-    static constexpr size_t kRowBytes = kRow * sizeof(cpx<R>);
-    static constexpr bool kShared = true;
-    cpx<R>* ring;
-    uint64_t* full;
-    uint64_t* empty;
-    uint32_t row0;
-    int32_t* err;
-    volatile int* abort;   // CTA-wide: set by the first wait that gives up
-    // In-line producer (one thread of the CTA when there is no producer
-    // warp): before taking row r it issues rows up to r + S - 1, waiting only
-    // for rows it needs itself (<= r) and skipping ahead rows whose slot is
-    // still held.
-    bool producer;
-    const char* src;       // key rows in global memory
-    uint32_t total;        // rows to stream
-    uint32_t next_issue;   // first row not issued yet
-
-    __device__ __forceinline__ void give_up() {
-        *abort = 1;
-        atomicExch(err, 3);
-    }
-    __device__ __forceinline__ void issue_one() {
-        const uint32_t slot = next_issue % S;
-        mbar_arrive_expect_tx(&full[slot], (uint32_t)kRowBytes);
-        bulk_copy_g2s(reinterpret_cast<char*>(ring) + slot * kRowBytes,
-                      src + (size_t)next_issue * kRowBytes, (uint32_t)kRowBytes, &full[slot]);
-        ++next_issue;
-    }
-    __device__ __forceinline__ void issue_upto(uint32_t r) {
-        while (next_issue < total && next_issue < r + S) {
-            const uint32_t slot = next_issue % S;
-            if (next_issue >= S) {
-                const uint32_t parity = ((next_issue / S) - 1) & 1;
-                if (next_issue <= r) {
-                    if (!mbar_wait_bounded(&empty[slot], parity, abort)) {
-                        give_up();
-                        next_issue = total;  // stop streaming; consumers give up and finish
-                        return;
-                    }
-                } else if (!mbar_try_wait(&empty[slot], parity)) {
-                    return;
-                }
-            }
-            issue_one();
-        }
-    }
-    // Issue rows up to r + S - 1 whose slots are free, without waiting.
-    __device__ __forceinline__ void issue_ready(uint32_t r) {
-        while (next_issue < total && next_issue < r + S) {
-            if (next_issue >= S && !mbar_try_wait(&empty[next_issue % S], ((next_issue / S) - 1) & 1)) return;
-            issue_one();
-        }
-    }
-    // Issue every row up to `last` (inclusive), waiting for their slots: used
-    // before the producer blocks on another group, for rows that group needs.
-    // Deadlock-free as long as the rows whose slots are reused (<= last - S)
-    // are released by consumers that need only rows already issued.
-    __device__ __forceinline__ void issue_through(uint32_t last) {
-        while (next_issue < total && next_issue <= last) {
-            if (next_issue >= S &&
-                !mbar_wait_bounded(&empty[next_issue % S], ((next_issue / S) - 1) & 1, abort)) {
-                give_up();
-                next_issue = total;
-                return;
-            }
-            issue_one();
-        }
-    }
-    // wait until every issued copy has landed (end of kernel)
-    __device__ __forceinline__ void drain() {
-        for (uint32_t r = next_issue > S ? next_issue - S : 0; r < next_issue; ++r)
-            if (!mbar_wait_bounded(&full[r % S], (r / S) & 1)) atomicExch(err, 3);
-    }
-    __device__ __forceinline__ void prefetch(int, int, int) const {}
-    __device__ __forceinline__ const cpx<R>* acquire(int p) {
-        const uint32_t r = row0 + (uint32_t)p;
-        if (producer) issue_upto(r);
-        const uint32_t slot = r % S;
-        if (!mbar_wait_bounded(&full[slot], (r / S) & 1, abort)) give_up();
-        return ring + slot * kRow;
-    }
-    __device__ __forceinline__ void release(int p) const { mbar_arrive(&empty[(row0 + (uint32_t)p) % S]); }
-};
-
-// The lane-pair kernel's way to the rows: acquire() in two parts, so that the
-// arrival test's round trip overlaps other work -- poll() issues rows whose
-// slots are free (producer, without waiting) and tests once whether row p has
-// landed, acquire_polled() issues and waits (bounded) only if it had not --
-// and one lane releases a slot for its whole warp (the slot's count is the
-// number of consumer warps).
-template <typename R, int PARTS, int S>
-struct PolledRingKeys : RingKeys<R, PARTS, S> {
-    using Base = RingKeys<R, PARTS, S>;
-    __device__ __forceinline__ bool poll(int p) {
-        const uint32_t r = this->row0 + (uint32_t)p;
-        if (this->producer) this->issue_ready(r);
-        __syncwarp();
-        return mbar_try_wait(&this->full[r % S], (r / S) & 1);
-    }
-    __device__ __forceinline__ const cpx<R>* acquire_polled(int p, bool landed) {
-        const uint32_t r = this->row0 + (uint32_t)p;
-        const uint32_t slot = r % S;
-        if (!landed) {
-            if (this->producer) this->issue_upto(r);
-            if (!mbar_wait_bounded(&this->full[slot], (r / S) & 1, this->abort)) this->give_up();
-        }
-        __syncwarp();
-        return this->ring + slot * Base::kRow;
-    }
-    __device__ __forceinline__ void release(int p) const {
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) mbar_arrive(&this->empty[(this->row0 + (uint32_t)p) % S]);
-    }
-};
-
 template <typename R, int PARTS, int GROUPS, int L, int S, int NB = 1>
 struct RingPlan {
     static constexpr size_t kRowBytes = (size_t)2 * PARTS * kHalf * sizeof(cpx<R>);
@@ -953,15 +835,12 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
     const int warp = threadIdx.x >> 5;
     const int n = kp.n;
     const uint32_t total_rows = (uint32_t)n * kpl;
-    RingKeys<R, PARTS, S> keys{ring, full, empty, 0, a.err, abort, false,
+    RingKeys<R, PARTS, S, !INLINE> keys{ring, full, empty, 0, a.err, abort, false,
                                reinterpret_cast<const char*>(a.gsw), total_rows, 0};
     if (!INLINE && warp == 2 * GROUPS) {
         // producer warp: one lane streams all n * 2l key rows in order
         if ((threadIdx.x & 31) == 0 && !a.stall_keys) {
-            for (uint32_t r = 0; r < total_rows; ++r) {
-                keys.issue_upto(r);  // blocks on row r's slot, issues up to r + S - 1
-                if (keys.next_issue <= r) break;  // timed out
-            }
+            keys.issue_through(total_rows - 1);
             keys.drain();
         }
         return;
@@ -2432,7 +2311,10 @@ __device__ __forceinline__ void ep_step_half(const StepCtx<R, PARTS, 1>& S, Keys
     }
     pair_sync(pair_bar);
     // the next step's first rows land during this step's inverse transforms
-    if (keys.producer) keys.issue_upto(keys.row0 + 2 * L - 1);
+    if (keys.producer) {
+        keys.stop_if(*keys.abort);  // the other half has given up on a row
+        keys.issue_upto(keys.row0 + 2 * L - 1);
+    }
     {
         const cpx<R>* inbox = S.s[0].b0;
 #pragma unroll

@@ -16,11 +16,11 @@ def model(tmp_path_factory):
     if not shutil.which("g++"):
         pytest.skip("no g++")
     exe = str(tmp_path_factory.mktemp("streams") / "key_streams")
-    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, "-o", exe, os.path.join(HERE, "key_streams.cpp")],
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", CSRC, "-o", exe, os.path.join(HERE, "key_streams.cpp")],
                    check=True, capture_output=True)
 
     def run(what, lost):
-        return subprocess.run([exe, what, str(lost)], capture_output=True, text=True).stdout.split("\n")[:-1]
+        return subprocess.run([exe, what, str(lost)], capture_output=True, text=True, timeout=60).stdout.split("\n")[:-1]
 
     return run
 
@@ -29,4 +29,11 @@ def model(tmp_path_factory):
 @pytest.mark.parametrize("stream,rows", [("products2", 12), ("products3", 18)])
 def test_product_stream_ends_by_itself(model, stream, rows):
     for lost in (-1, 0, 3, 6, rows - 2, rows - 1):
+        assert model(stream, lost) == [], lost
+
+
+# shared rings: streamed in line, by a producer warp, for lane pairs, for two halves
+@pytest.mark.parametrize("stream", ["ring", "producer_warp", "lane_pairs", "pair"])
+def test_ring_ends_by_itself(model, stream):
+    for lost in (-1, 0, 2, 4, 9, 13, 16, 17):
         assert model(stream, lost) == [], lost
