@@ -221,13 +221,14 @@ __device__ __forceinline__ FftTwiddles<R> hot_twiddles(const cpx<R>* hot) {
 // (fft512_forward_tw_multi), and IB parts of an output polynomial are
 // transformed back together.
 // ----------------------------------------------------------------------
-template <typename R, int PARTS, int NB>
+template <typename R, int PARTS, int NB, typename Bar = int>
 struct StepCtx {
     FftTwiddles<R> tw;  // smem twiddles: a = psi^t W^(tq) (twist folded), b = W^(8jq)
     FftIdx ix;          // this thread's exchange slots
     FftScratch<R> s[NB];
     int32_t* acc;       // smem 2 x N
-    int t, bar_id;
+    int t;
+    Bar bar_id;
     int Bgbit, split;
     uint32_t offset;
 };
@@ -282,8 +283,8 @@ __device__ __forceinline__ void mac_row(cpx<R> (&out)[2][PARTS][8], const cpx<R>
 
 // The L levels of input polynomial jp: digits, forward transforms run
 // together, and their key rows multiply-accumulated.
-template <int L, typename R, int PARTS, int NB, typename Keys>
-__device__ __forceinline__ void forward_levels(const StepCtx<R, PARTS, NB>& S, Keys& keys,
+template <int L, typename R, int PARTS, int NB, typename Bar, typename Keys>
+__device__ __forceinline__ void forward_levels(const StepCtx<R, PARTS, NB, Bar>& S, Keys& keys,
                                                cpx<R> (&out)[2][PARTS][8], const uint32_t (&r0)[8],
                                                const uint32_t (&r1)[8], int p0, uint32_t mask, int halfBg) {
     const int t = S.t;
@@ -301,8 +302,8 @@ __device__ __forceinline__ void forward_levels(const StepCtx<R, PARTS, NB>& S, K
     }
 }
 
-template <typename R, int PARTS, bool ROT, int L, int IB, int NB, typename Keys>
-__device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB>& S, Keys& keys, int a) {
+template <typename R, int PARTS, bool ROT, int L, int IB, int NB, typename Bar, typename Keys>
+__device__ __forceinline__ void ep_step(const StepCtx<R, PARTS, NB, Bar>& S, Keys& keys, int a) {
     static_assert(PARTS % IB == 0 && L <= NB && IB <= NB, "batch sizes");
     const int t = S.t;
     const int halfBg = 1 << (S.Bgbit - 1);
@@ -537,7 +538,7 @@ struct KParams {
 template <typename R, int PARTS, int MODE, int GROUPS, int L>
 __global__ void __launch_bounds__(64 * GROUPS, 1) k_external_product(KParams kp, Tables T, EpArgs a) {
     constexpr int NB = L > PARTS ? L : PARTS;
-    using Ctx = StepCtx<R, PARTS, NB>;
+    using Ctx = StepCtx<R, PARTS, NB, ConvergedBarrier>;
     using Plan = SmemPlan<R, NB>;
     extern __shared__ __align__(128) char smem[];
     cpx<R>* tables = reinterpret_cast<cpx<R>*>(smem);
@@ -562,7 +563,7 @@ __global__ void __launch_bounds__(64 * GROUPS, 1) k_external_product(KParams kp,
     for (int b = 0; b < NB; ++b)
         S.s[b] = scratch_at<R>(gbase + Plan::acc + (size_t)b * 2 * kScratchStride * sizeof(cpx<R>));
     S.t = t;
-    S.bar_id = 1 + g;
+    S.bar_id = {1 + g};
     S.Bgbit = kp.Bgbit;
     S.split = kp.split;
     S.offset = kp.offset;
@@ -2252,14 +2253,12 @@ __global__ void __launch_bounds__(128 * L, 1) k_blind_rotate_spread_f64(KParams 
 // small batches, single gates).  Key rows come through the same shared ring
 // as k_blind_rotate_ring; each row is read by one half of every ciphertext.
 // ----------------------------------------------------------------------
-__device__ __forceinline__ void pair_sync(int bar_id) {
-    asm volatile("barrier.sync %0, %1;" ::"r"(bar_id), "r"(2 * kFftThreads) : "memory");
-}
+__device__ __forceinline__ void pair_sync(int bar_id) { converged_sync(bar_id, 2 * kFftThreads); }
 
 // h is the half; out[h] and out[1 - h] are picked by uniform branches so
 // that the accumulators stay in registers with one copy of the code.
 template <typename R, int PARTS, int L, typename Keys>
-__device__ __forceinline__ void ep_step_half(const StepCtx<R, PARTS, 1>& S, Keys& keys, int a, int h,
+__device__ __forceinline__ void ep_step_half(const StepCtx<R, PARTS, 1, ConvergedBarrier>& S, Keys& keys, int a, int h,
                                              cpx<R>* peer_inbox, int pair_bar) {
     const int t = S.t;
     const int halfBg = 1 << (S.Bgbit - 1);
@@ -2393,14 +2392,14 @@ __global__ void __launch_bounds__(128 * PAIRS, 1) k_blind_rotate_pair(KParams kp
                                reinterpret_cast<const char*>(a.gsw), (uint32_t)n * kpl, 0};
 
     char* pbase = smem + Plan::pair_off + (size_t)pr * Plan::pair;
-    StepCtx<R, PARTS, 1> St;
+    StepCtx<R, PARTS, 1, ConvergedBarrier> St;
     St.tw = hot_twiddles<R>(tables);
     St.ix = make_fft_idx(t);
     St.acc = reinterpret_cast<int32_t*>(pbase);
     St.s[0] = scratch_at<R>(pbase + Plan::acc + h * Plan::half_scratch);
     cpx<R>* peer_inbox = reinterpret_cast<cpx<R>*>(pbase + Plan::acc + (1 - h) * Plan::half_scratch);
     St.t = t;
-    St.bar_id = 1 + 2 * pr + h;
+    St.bar_id = {1 + 2 * pr + h};
     const int pair_bar = 1 + 2 * PAIRS + pr;
     St.Bgbit = kp.Bgbit;
     St.split = kp.split;

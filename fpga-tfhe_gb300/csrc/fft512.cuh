@@ -266,6 +266,19 @@ __device__ __forceinline__ cpx<double> dft8_one(const cpx<double> (&v)[8], bool 
 __device__ __forceinline__ void group_sync(int bar_id) {
     asm volatile("barrier.sync %0, %1;" ::"r"(bar_id), "r"(kFftThreads) : "memory");
 }
+// The same barrier with the warp brought together first, as its aligned form
+// needs.  Faster in the L2-direct kernel, whose warps are together anyway (one
+// ciphertext, l = 2: 1.84 -> 1.76 ms), and in the pair kernel (three per CTA
+// 6.46 -> 5.05 ms, two 3.25 -> 3.22 ms); slower in the rings (4-per-SM wave
+// 4.57 -> 4.65 ms, 3 per SM 4.21 -> 4.32 to 4.42 ms).
+struct ConvergedBarrier {
+    int id;
+};
+__device__ __forceinline__ void converged_sync(int bar_id, int threads) {
+    __syncwarp();
+    asm volatile("barrier.sync.aligned %0, %1;" ::"r"(bar_id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void group_sync(ConvergedBarrier bar) { converged_sync(bar.id, kFftThreads); }
 
 // Two ping-pong exchange buffers of kScratchStride interleaved complex values.
 template <typename R>
@@ -407,10 +420,10 @@ __device__ __forceinline__ cpx<R> twist_c(int r) {
 // of the transform of the twisted sequence.  tw.a = psi^t W^(tq) table.
 // With NB > 1 every twiddle is loaded once and applied to all NB point sets
 // (the compiler cannot merge the loads across the exchange stores).
-template <int NB, typename R>
+template <int NB, typename R, typename Bar>
 __device__ __forceinline__ void fft512_forward_tw_multi(cpx<R> (&v)[NB][8], const FftScratch<R> (&s)[NB],
                                                         const FftTwiddles<R>& tw, const FftIdx& ix, int t,
-                                                        int bar_id) {
+                                                        Bar bar_id) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
 #pragma unroll
@@ -456,10 +469,10 @@ __device__ __forceinline__ void fft512_forward_tw_multi(cpx<R> (&v)[NB][8], cons
 
 // In: v[q] = position 8t + q.  Out: v[q] = 512 z[t + 64q] untwisted (times
 // psi^-(t + 64q)), not yet divided by 512.
-template <int NB, typename R>
+template <int NB, typename R, typename Bar>
 __device__ __forceinline__ void fft512_inverse_tw_multi(cpx<R> (&v)[NB][8], const FftScratch<R> (&s)[NB],
                                                         const FftTwiddles<R>& tw, const FftIdx& ix, int t,
-                                                        int bar_id) {
+                                                        Bar bar_id) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         dft8<-1>(v[b]);
@@ -500,18 +513,18 @@ __device__ __forceinline__ void fft512_inverse_tw_multi(cpx<R> (&v)[NB][8], cons
     }
 }
 
-template <typename R>
+template <typename R, typename Bar>
 __device__ __forceinline__ void fft512_forward_tw(cpx<R> (&v)[8], const FftScratch<R>& s,
                                                   const FftTwiddles<R>& tw, const FftIdx& ix, int t,
-                                                  int bar_id) {
+                                                  Bar bar_id) {
     fft512_forward_tw_multi<1>(*reinterpret_cast<cpx<R>(*)[1][8]>(&v),
                                *reinterpret_cast<const FftScratch<R>(*)[1]>(&s), tw, ix, t, bar_id);
 }
 
-template <typename R>
+template <typename R, typename Bar>
 __device__ __forceinline__ void fft512_inverse_tw(cpx<R> (&v)[8], const FftScratch<R>& s,
                                                   const FftTwiddles<R>& tw, const FftIdx& ix, int t,
-                                                  int bar_id) {
+                                                  Bar bar_id) {
     fft512_inverse_tw_multi<1>(*reinterpret_cast<cpx<R>(*)[1][8]>(&v),
                                *reinterpret_cast<const FftScratch<R>(*)[1]>(&s), tw, ix, t, bar_id);
 }
