@@ -1176,6 +1176,8 @@ def launched_blind_rotations(form, shape, batch, l=3):
         two, one = "k_blind_rotate_spread2<%d" % l + tail, "k_blind_rotate_spread<%d" % l + tail
         if cnt <= SMS // 2:
             return [two + " x %d" % cnt]
+        if pair and l == 2 and cnt > SMS + SMS // 2:
+            return ["k_blind_rotate_pair<float,2,2,2,4> x %d" % cnt]
         if SMS < cnt <= SMS + SMS // 2:
             return [one + " x %d" % SMS, two + " x %d" % (cnt - SMS)]
         return [one + " x %d" % cnt]

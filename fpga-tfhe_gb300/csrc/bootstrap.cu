@@ -2929,11 +2929,15 @@ cudaError_t launch_ring_pairs(const DevParams& P, const Tables& T, const EpArgs&
 
 // Up to two ciphertexts per SM: one per cluster of two SMs up to half as many
 // as SMs, one per CTA up to as many, and two launches (a wave of one per CTA,
-// then the rest) above.
+// then the rest) above.  In the pair kernel's order with l = 2 the pair kernel
+// itself is the faster one from 1.5 per SM on (1.93 ms for 229 to 304, where
+// two waves of one per CTA take 2.01 to 2.03 ms; l = 3: 3.22 against 3.05 ms;
+// 220 with l = 2 1.80 ms in two launches).
 template <int L, bool PAIR>
 cudaError_t launch_low_latency(const DevParams& P, const Tables& T, const EpArgs& a, cudaStream_t st) {
     if (a.count <= kSmCount / 2) return launch_spread2<L, PAIR>(P, T, a, st);
     const int rest = a.count - kSmCount;
+    if (PAIR && L == 2 && rest > kSmCount / 2) return launch_pair_fp32<L>(P, T, a, 2, st);
     if (rest <= 0 || rest > kSmCount / 2) return launch_spread<L, PAIR>(P, T, a, st);
     const cudaError_t e = launch_spread<L, PAIR>(P, T, slice_blind_rotate(P, a, 0, kSmCount), st);
     if (e != cudaSuccess) return e;

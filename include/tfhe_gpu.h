@@ -104,7 +104,7 @@ size_t tfhe_gpu_device_bytes(const tfhe_gpu_ctx* ctx);
  *   0 = automatic: whole waves of 6 ciphertexts per SM on shape 10; a
  *       remainder of at most one per two SMs on shape 16, of at most 1 per
  *       SM on shape 14, of at most 2 per SM on these two in the pair kernel's
- *       summation order, of at most 4 per SM as one shape-9 wave, of at most
+ *       summation order (l = 2 above 1.5 per SM: on that kernel), of at most 4 per SM as one shape-9 wave, of at most
  *       5 per SM as a full shape-9 wave and the rest by the rules before,
  *       else one more shape-10 wave;
  *   1, 2, 4 = ciphertexts (64 threads each) per CTA, key rows read from L2
