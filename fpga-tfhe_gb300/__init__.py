@@ -562,9 +562,9 @@ class Engine:
         return lwe, tlwe, ks, bk
 
     def selftest_timeout(self, form, count):
-        """Status of a blind rotation whose key stream never starts (the
-        bounded waits run out): 3 = TFHE_GPU_TIMEOUT, 0 for shapes without
-        waits."""
+        """Status of a blind rotation whose copies of key rows are never started
+        (the bounded waits run out): 3 = TFHE_GPU_TIMEOUT, 0 for shapes that
+        read key rows from L2."""
         return self.lib.tfhe_gpu_selftest_timeout(self.ctx, self._form(form), int(count))
 
     def selftest_timeout_in(self, part, count):

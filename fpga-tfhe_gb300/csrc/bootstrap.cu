@@ -1252,11 +1252,59 @@ __device__ __forceinline__ void rotated_pair(const int32_t* acc, int j, int t, i
     r1 = ((uint32_t)w.y ^ m) - (uint32_t)p.y + (offset - m);
 }
 
+// The producer warp of k_blind_rotate_spread: the key values of every step into
+// the one buffer, as soon as the owners have used the last step's.  Owners that
+// have given up on a step free its values too, so the producer waits for the
+// last copy itself before it fills the buffer again.
+// EARLY arms the barrier and prefetches before the owners are done: 263
+// ciphertexts in the pair kernel's order with l = 3 3.06 -> 3.04 ms; in the other
+// forms it is slower (152 ciphertexts 1.560 -> 1.583 ms).
+template <int L, bool EARLY>
+__device__ __forceinline__ void spread_stream(const EpArgs& a, char* smem, uint64_t* kfull, uint64_t* kfree,
+                                              volatile int* abort, int n, int c) {
+    using Plan = SpreadPlan<L>;
+    constexpr int kRows = 2 * L;
+    constexpr uint32_t kPart = kHalf * sizeof(cpx<float>);
+    const int u = threadIdx.x & 31;
+    const char* gsw = reinterpret_cast<const char*>(a.gsw);  // parts lie in order, row by row
+    constexpr size_t kStep = (size_t)Plan::kKeyParts * kPart, kRowBytes = kStep / kRows;
+    const auto prefetch = [&](int i) {  // rows into L2 two steps ahead of their copies
+        if (i + 2 < n && u < kRows) bulk_prefetch_l2(gsw + (size_t)(i + 2) * kStep + u * kRowBytes, kRowBytes);
+    };
+    uint32_t k = 0;  // steps copied
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+        if (EARLY) prefetch(i);
+        bool go = k == 0 || mbar_wait_bounded(kfull, (k - 1) & 1, abort);
+        if (EARLY) {
+            go = __all_sync(0xffffffffu, go);
+            if (u == 0 && go) mbar_arrive_expect_tx(kfull, (uint32_t)kStep);
+        }
+        go = go && (k == 0 || mbar_wait_bounded(kfree, (k - 1) & 1, abort));
+        go = __all_sync(0xffffffffu, go);
+        if (!go) {
+            *abort = 1;
+            atomicExch(a.err, 3);
+            break;
+        }
+        if (!EARLY) {
+            if (u == 0) mbar_arrive_expect_tx(kfull, (uint32_t)kStep);
+            __syncwarp();
+        }
+        if (u < Plan::kKeyParts && !a.stall_keys)
+            bulk_copy_g2s(smem + Plan::key_off + (size_t)u * Plan::kKeyPart, gsw + (size_t)i * kStep + u * kPart,
+                          kPart, kfull);
+        if (!EARLY) prefetch(i);
+        ++k;
+    }
+    // no copy in flight at the end of the kernel
+    if (k > 0 && !mbar_wait_bounded(kfull, (k - 1) & 1)) atomicExch(a.err, 3);
+    __syncwarp();
+}
+
 template <int L, bool PAIR>
 __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spread(KParams kp, Tables T, EpArgs a) {
     using Plan = SpreadPlan<L>;
-    constexpr int kRows = 2 * L;
-    constexpr int kRowElems = 2 * 2 * kHalf;  // complex values per key row
     extern __shared__ __align__(128) char smem[];
     cpx<float>* tables = reinterpret_cast<cpx<float>*>(smem);
     int32_t* acc = reinterpret_cast<int32_t*>(smem + Plan::acc_off);
@@ -1291,36 +1339,11 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
     }
     __syncthreads();
 
-    const cpx<float>* gsw = reinterpret_cast<const cpx<float>*>(a.gsw);
-    const size_t step_elems = (size_t)kRows * kRowElems;
     const auto gave_up = [&]() {
         *abort = 1;
         atomicExch(a.err, 3);
     };
-    if (set == Plan::kSets) {
-        const int u = threadIdx.x & 31;
-        const cpx<float>* src = gsw + (size_t)u * kHalf;  // parts lie in order, row by row
-        int i = 0;
-#pragma unroll 1
-        for (; i < n; ++i) {
-            if (i > 0 && !mbar_wait_bounded(kfree, (uint32_t)(i - 1) & 1, abort)) {
-                gave_up();
-                break;
-            }
-            __syncwarp();
-            if (u == 0) mbar_arrive_expect_tx(kfull, (uint32_t)(Plan::kKeyParts * kHalf * sizeof(cpx<float>)));
-            __syncwarp();
-            if (u < Plan::kKeyParts)
-                bulk_copy_g2s(smem + Plan::key_off + (size_t)u * Plan::kKeyPart, src + (size_t)i * step_elems,
-                              (uint32_t)(kHalf * sizeof(cpx<float>)), kfull);
-            if (i + 2 < n && u < kRows)  // rows into L2 ahead of their copies
-                bulk_prefetch_l2(gsw + (size_t)(i + 2) * step_elems + (size_t)u * kRowElems,
-                                 kRowElems * sizeof(cpx<float>));
-        }
-        // no copy in flight at the end of the kernel
-        if (!mbar_wait_bounded(kfull, (uint32_t)(i - 1) & 1)) atomicExch(a.err, 3);
-        __syncwarp();
-    } else {
+    if (set != Plan::kSets) {
         // barrier of all sets (the producer warp takes no part)
         const auto step_sync = []() {
             asm volatile("barrier.sync 15, %0;" ::"n"(kDuoThreads * Plan::kSets) : "memory");
@@ -1344,16 +1367,18 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
         const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
         const int32_t* rot = bara ? bara : xs;
         int32_t rot_next = rot[0];
+        uint32_t k = 0;  // parity of the step
 #pragma unroll 1
         for (int i = 0; i < n; ++i) {
             const int ai = bara ? rot_next : mod_switch_2n(rot_next);
             if (i + 1 < n) rot_next = rot[i + 1];
             if (ai == 0) {  // tfhe_blindRotate_FFT.cpp:114 (uniform over the CTA): the keys go by unused
                 if (owner) {
-                    if (!mbar_wait_bounded(kfull, (uint32_t)i & 1, abort)) gave_up();
+                    if (!mbar_wait_bounded(kfull, k, abort)) gave_up();
                     __syncwarp();
                     if ((threadIdx.x & 31) == 0) mbar_arrive(kfree);
                 }
+                k ^= 1;
                 continue;
             }
             cpx<float> v[1][8];
@@ -1372,7 +1397,7 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
             }
             step_sync();  // every D in place; every read of acc done
             if (owner) {
-                if (!mbar_wait_bounded(kfull, (uint32_t)i & 1, abort)) gave_up();
+                if (!mbar_wait_bounded(kfull, k, abort)) gave_up();
                 __syncwarp();
                 cpx<float> o[1][8];
 #pragma unroll
@@ -1381,7 +1406,7 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
 #pragma unroll
                 for (int q = 0; q < 8; ++q) other[q] = {0.f, 0.f};
 #pragma unroll
-                for (int qq = 0; qq < 4; ++qq)
+                for (int qq = 0; qq < 4; ++qq) {
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
                         float4 w[L];
@@ -1403,9 +1428,10 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
                                          h ? cpx<float>{w[2].z, w[2].w} : cpx<float>{w[2].x, w[2].y});
                         }
                     }
-                if constexpr (PAIR) {
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) o[0][q] = cadd(o[0][q], other[q]);
+                    if constexpr (PAIR) {
+                        o[0][2 * qq] = cadd(o[0][2 * qq], other[2 * qq]);
+                        o[0][2 * qq + 1] = cadd(o[0][2 * qq + 1], other[2 * qq + 1]);
+                    }
                 }
                 __syncwarp();
                 if ((threadIdx.x & 31) == 0) mbar_arrive(kfree);
@@ -1423,8 +1449,11 @@ __global__ void __launch_bounds__(SpreadPlan<L>::kThreads, 1) k_blind_rotate_spr
                     spread_put<L>(acc, set, t + 64 * q + e * kHalf, own[q]);
                 }
             }
+            k ^= 1;
             step_sync();  // the accumulator is updated before the next step reads it
         }
+    } else {
+        spread_stream<L, (L == 3 && PAIR)>(a, smem, kfull, kfree, abort, n, c);
     }
     __syncthreads();
     if (a.acc_out) {

@@ -103,7 +103,7 @@ tfhe_gpu_status check_device_status(tfhe_gpu_ctx* ctx) {
     CK(ctx, cudaMemcpy(&v, ctx->d_err, sizeof(v), cudaMemcpyDeviceToHost));
     if (v == 0) return TFHE_GPU_OK;
     CK(ctx, cudaMemset(ctx->d_err, 0, sizeof(int32_t)));
-    return fail(ctx, TFHE_GPU_TIMEOUT, "a bounded wait in a kernel gave up (key-row ring stalled)");
+    return fail(ctx, TFHE_GPU_TIMEOUT, "a bounded wait in a kernel gave up (a copy or a store between SMs did not arrive)");
 }
 
 // The end of a host-buffer call: `bytes` of results at d_out to `out`, the

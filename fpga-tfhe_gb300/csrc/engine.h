@@ -80,8 +80,9 @@ struct EpArgs {
     // tv + c * tv_stride) instead of the constant mu; nullptr = constant mu
     const int32_t* tv;
     int32_t tv_stride;
-    // self-test of the bounded waits: the key-row ring's producer issues
-    // nothing, so every consumer wait runs out (tfhe_gpu_selftest_timeout)
+    // self-test of the bounded waits (tfhe_gpu_selftest_timeout): kernels that
+    // copy key rows into shared memory start none of the copies, so every wait
+    // for them runs out
     int32_t stall_keys;
 };
 

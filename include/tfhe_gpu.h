@@ -325,12 +325,13 @@ tfhe_gpu_status tfhe_gpu_bootsGates_noalloc(tfhe_gpu_ctx* ctx, const int32_t* ga
                                             tfhe_gpu_form form, void* stream);
 
 /* Self-test of the device-side failure path: runs one blind rotation of
- * `count` samples with the current launch shape of `form` whose key-row
- * stream is never started, so every bounded wait in the kernel runs out
+ * `count` samples with the current launch shape of `form` without the copies
+ * of key rows into shared memory, so every bounded wait for them runs out
  * (after about 2 s; the first one to give up tells the rest of its CTA to
- * stop waiting).  Returns what the host sees: TFHE_GPU_TIMEOUT for the
- * shared-ring shapes; TFHE_GPU_OK for the L2-direct shapes, which have no
- * waits.  The context stays usable.  No counterpart in the reference. */
+ * stop waiting).  Returns what the host sees: TFHE_GPU_TIMEOUT for the shapes
+ * that copy key rows (the rings, the pair kernel and the one-per-CTA
+ * split-FP32 kernel); TFHE_GPU_OK for those that read them from L2.  The
+ * context stays usable.  No counterpart in the reference. */
 tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form, int32_t count);
 /* The same for another part of the engine, over `count` samples:
  *   TFHE_GPU_PART_KEY_SWITCH: a key switch whose table stream ends after its

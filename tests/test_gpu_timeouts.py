@@ -42,3 +42,31 @@ def test_key_switch_timeout(pkg, torch_cuda, count):
         _timeout_then(lambda: e.selftest_timeout_in("key_switch", count), check)
     finally:
         e.close()
+
+
+# one-per-CTA split-FP32 kernel: by its own shape, by batch size, in two waves and in the pair kernel's order
+@pytest.mark.parametrize("params,shape,count", [("default", 14, 2), ("default", 0, 77), ("stress", 15, 304),
+                                                ("default", 0, 230)])
+def test_one_per_cta_rotation_timeout(pkg, torch_cuda, params, shape, count):
+    torch = torch_cuda
+    e = pkg.Engine(pkg.default_params() if params == "default" else pkg.stress_params())
+    try:
+        e.gate_keyset([9], forms=("split_fp32",), want_bk=False)
+        x = torch.randint(-2 ** 31, 2 ** 31, (count, e.params.n + 1), device="cuda", dtype=torch.int32)
+        out = torch.empty((2, count, 1025), device="cuda", dtype=torch.int32)
+        sp = torch.cuda.current_stream().cuda_stream
+        e.set_groups_per_cta("split_fp32", shape)
+
+        def bootstrap(k):
+            e.tfhe_bootstrap_woKS_FFT(out[k], x, 1 << 29, count, "split_fp32", stream=sp)
+            torch.cuda.synchronize()
+            e.synchronize()
+
+        def check():
+            bootstrap(1)
+            assert torch.equal(out[0], out[1])
+
+        bootstrap(0)
+        _timeout_then(lambda: e.selftest_timeout("split_fp32", count), check)
+    finally:
+        e.close()
