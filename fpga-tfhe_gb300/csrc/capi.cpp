@@ -920,7 +920,8 @@ tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form,
     RET(ensure_scratch(ctx, 0, (size_t)count * (n + 1) * sizeof(int32_t), &x));
     RET(ensure_scratch(ctx, 1, (size_t)count * (nk + 1) * sizeof(int32_t), &u));
     cudaStream_t st = ctx->stream;
-    CK(ctx, cudaMemsetAsync(x, 0, (size_t)count * (n + 1) * sizeof(int32_t), st));
+    // samples that take every step (a step with a_i = 0 waits for no key)
+    CK(ctx, cudaMemsetAsync(x, 0x55, (size_t)count * (n + 1) * sizeof(int32_t), st));
     EpArgs a{};
     a.err = ctx->d_err;
     a.x = (const int32_t*)x;

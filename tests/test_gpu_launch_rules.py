@@ -52,3 +52,18 @@ def test_two_per_sm_with_two_levels_is_not_slower_than_the_pair_kernel(pkg, torc
         assert _bootstrap_us(torch, e, 0, x) < 1.025 * _bootstrap_us(torch, e, 12, x)
     finally:
         e.close()
+
+
+# one ciphertext per CTA
+@pytest.mark.parametrize("count", [152])
+def test_noiseless_constants_cost_no_steps(pkg, torch_cuda, count):
+    """Samples with no mask (bootsCONSTANT) rotate by nothing: no step is taken
+    and no key is copied for them."""
+    torch = torch_cuda
+    e = _engine(pkg, "default")
+    try:
+        x = _uniform(torch, count, e.params.n + 1)
+        zero = torch.zeros_like(x)
+        assert _bootstrap_us(torch, e, 0, zero) < 0.2 * _bootstrap_us(torch, e, 0, x)
+    finally:
+        e.close()
