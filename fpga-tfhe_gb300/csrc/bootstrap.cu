@@ -647,13 +647,15 @@ __global__ void __launch_bounds__(64 * GROUPS, 1) k_external_product(KParams kp,
 // through registers: 34.1 -> 27.1 us for 1,024 products of the default set
 // (4.3 TB/s), 83.4 -> 59.7 us for 3,000 (5.8 TB/s), 14.5 -> 10.4 us for 300.
 // What is left at 1,024 is the last round of 2.7 groups per SM.
+// A MuxRotate item with rotation 0 is a copy of its sample and streams no row
+// (3,000 of them 54 -> 10.5 us; with all rows 96 KB each).
 // The arithmetic is ep_step's, bit for bit.
 // ----------------------------------------------------------------------
 template <int L>
 struct ProductPlan {
     static constexpr int kGroups = 4;
-    static constexpr int S = ItemKeys<L>::S;
-    static constexpr size_t kRowBytes = ItemKeys<L>::kRowBytes;
+    static constexpr int S = ItemKeys<L, false>::S;
+    static constexpr size_t kRowBytes = ItemKeys<L, false>::kRowBytes;
     static constexpr size_t ring_off = (kHotSize * sizeof(cpx<float>) + 127) & ~(size_t)127;
     static constexpr size_t x_off = ring_off + kGroups * S * kRowBytes;
     static constexpr size_t x_group = 4 * kScratchStride * sizeof(cpx<float>);  // two transforms, two buffers each
@@ -662,8 +664,8 @@ struct ProductPlan {
     static constexpr size_t total = flag_off + 16;
 };
 
-template <int NBK, int L>
-__device__ __forceinline__ void product_levels(ItemKeys<L>& keys, cpx<float> (&out)[2][2][8], const uint32_t (&r0)[8],
+template <int NBK, int L, bool ROT>
+__device__ __forceinline__ void product_levels(ItemKeys<L, ROT>& keys, cpx<float> (&out)[2][2][8], const uint32_t (&r0)[8],
                                                const uint32_t (&r1)[8], cpx<float>* x0, const FftTwiddles<float>& tw,
                                                const FftIdx& ix, int t, int bar_id, int Bgbit, int lev0) {
     const uint32_t mask = (1u << Bgbit) - 1;
@@ -702,11 +704,20 @@ __global__ void __launch_bounds__(64 * ProductPlan<L>::kGroups, 1)
     const int stride = (int)gridDim.x * Plan::kGroups;
     const int first = (int)(blockIdx.x + gridDim.x * g);
     const int items = first < a.count ? (a.count - 1 - first) / stride + 1 : 0;
-    ItemKeys<L> keys{reinterpret_cast<cpx<float>*>(smem + Plan::ring_off + g * Plan::S * Plan::kRowBytes),
-                     full + g * Plan::S, a.err, abort,
-                     reinterpret_cast<const char*>(a.gsw) + (size_t)first * a.gsw_stride,
-                     (size_t)stride * a.gsw_stride, (uint32_t)items * 2 * L, 0, 0, t};
-    if (t == 0) keys.issue();  // the first rows travel while the tables load
+    ItemKeys<L, ROT> keys{reinterpret_cast<cpx<float>*>(smem + Plan::ring_off + g * Plan::S * Plan::kRowBytes),
+                          full + g * Plan::S, a.err, abort,
+                          reinterpret_cast<const char*>(a.gsw) + (size_t)first * a.gsw_stride,
+                          (size_t)stride * a.gsw_stride, a.bara + first, stride, items, t, 0, 0, 0, 0, 0};
+    int a_next = 0;
+    if (ROT && items > 0) {
+        // a rotated read waits for its rotation, so the sample travels before it is read
+        a_next = a.bara[first];
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.acc_in + (size_t)first * 2 * kN + 32 * t));
+    }
+    if (t == 0) {  // the first rows travel while the tables load
+        keys.start();
+        keys.issue();
+    }
     load_hot_tables<float>(tables, T);
     __syncthreads();
     if (items == 0) return;
@@ -720,19 +731,17 @@ __global__ void __launch_bounds__(64 * ProductPlan<L>::kGroups, 1)
         const int item = first + it * stride;
         const int32_t* acc = a.acc_in + (size_t)item * 2 * kN;
         int32_t* res = a.acc_out + (size_t)item * 2 * kN;
-        if (it + 1 < items)  // the next item's sample into L2, 128 bytes a thread
+        const int ai = a_next;
+        if (it + 1 < items) {  // the next item's sample into L2, 128 bytes a thread
             asm volatile("prefetch.global.L2 [%0];" ::"l"(acc + (size_t)stride * 2 * kN + 32 * t));
-        const int ai = ROT ? a.bara[item] : 0;
-        if (ROT && ai == 0) {  // tfhe_blindRotate_FFT.cpp:114 -- the sample as it is; its rows still pass through
+            if (ROT) a_next = a.bara[item + stride];
+        }
+        if (ROT && ai == 0) {  // tfhe_blindRotate_FFT.cpp:114 -- the sample as it is, without its rows
             int32_t keep[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) keep[i] = acc[t + 64 * i];
 #pragma unroll
             for (int i = 0; i < 32; ++i) res[t + 64 * i] = keep[i];
-            for (int p = 0; p < 2 * L; ++p) {
-                keys.wait(keys.used);
-                keys.release(1, bar_id);
-            }
             continue;
         }
         cpx<float> out[2][2][8];

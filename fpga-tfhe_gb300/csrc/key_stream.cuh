@@ -12,35 +12,57 @@
 
 namespace tfhe_gb300 {
 
-// Row stream of one group of 64 threads of k_products_stream: row r is row
-// r % 2l of the group's item r / 2l.  A slot is refilled as soon as both warps
-// of the group have used it.
+// Row stream of one group of 64 threads of k_products_stream: the 2l rows of
+// each of the group's items in turn; with ROT only of those whose rotation is
+// not 0, which are the ones that use them.  A slot is refilled as soon as both
+// warps of the group have used it.
 //
 // A wait that gives up ends the stream: its slot's copy has not landed, so the
 // slot may not be armed or filled again.  drain() then waits for the copies
 // that are out, so that none is in flight when the CTA ends.
-template <int L>
+template <int L, bool ROT>
 struct ItemKeys {
     static constexpr int S = 2;  // row slots per group
     static constexpr size_t kRow = (size_t)2 * 2 * 512;
     static constexpr size_t kRowBytes = kRow * sizeof(cpx<float>);
+    static constexpr uint32_t kStopped = 1u << 31;
     cpx<float>* ring;
     uint64_t* full;
     int32_t* err;
     volatile int* abort;
     const char* src;     // first item
     size_t item_stride;  // bytes from one item of the group to the next
-    uint32_t total, next, used;  // rows of the stream; issued (+ kStopped once the stream has stopped); read
-    static constexpr uint32_t kStopped = 1u << 31;
-    int t;
+    const int32_t* rot;  // rotation of the first item, rot_stride apart
+    int rot_stride;
+    int items, t;
+    uint32_t next, used;  // rows issued (+ kStopped once the stream has stopped), rows read
+    // thread 0: the row to issue, and the rotation of the item after its own
+    int item, row, ahead;
 
+    // thread 0, once: the first item
+    __device__ __forceinline__ void start() {
+        item = -1;
+        if (ROT && items > 0) ahead = rot[0];
+        next_item();
+    }
+    __device__ __forceinline__ void next_item() {
+        row = 0;
+        int a;
+        do {
+            ++item;
+            a = ahead;
+            if (ROT && item + 1 < items) ahead = rot[(size_t)(item + 1) * rot_stride];
+        } while (ROT && item < items && a == 0);
+    }
     // thread 0: rows up to used + S - 1 (all earlier uses of their slots are over)
     __device__ __forceinline__ void issue() {
-        for (; next < total && next < used + S; ++next) {
-            const uint32_t slot = next % S, item = next / (2 * L), row = next - item * (2 * L);
+        while (item < items && next < used + S) {
+            const uint32_t slot = next % S;
             mbar_arrive_expect_tx(&full[slot], (uint32_t)kRowBytes);
             bulk_copy_g2s(reinterpret_cast<char*>(ring) + slot * kRowBytes,
                           src + item * item_stride + row * kRowBytes, (uint32_t)kRowBytes, &full[slot]);
+            ++next;
+            if (++row == 2 * L) next_item();
         }
     }
     __device__ __forceinline__ const cpx<float>* wait(uint32_t r) {

@@ -50,6 +50,7 @@ static std::set<std::string> g_faults;
 static const char* g_base;
 static long g_lost = -1, g_copies = 0;
 static size_t g_row_bytes;
+static std::vector<long> g_rows;  // copied, in order
 static void fault(const char* what) { g_faults.insert(what); }
 static bool passed(const uint64_t* bar, uint32_t parity) { return ((uint32_t)g_bars[bar].phase & 1) != parity; }
 
@@ -98,6 +99,7 @@ inline void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* 
     if (g_out.count(dst)) fault("copy into a slot whose last copy has not landed");
     const long row = (static_cast<const char*>(src) - g_base) / (long)g_row_bytes;
     ++g_copies;
+    g_rows.push_back(row);
     if (row == g_lost) {
         g_out[dst] = bar;
         g_drained.erase(bar);
@@ -146,6 +148,7 @@ static void reset(long lost, size_t row_bytes, const char* base) {
     g_out.clear();
     g_drained.clear();
     g_copies = 0;
+    g_rows.clear();
     g_lost = lost;
     g_row_bytes = row_bytes;
     g_base = base;
@@ -171,10 +174,10 @@ static void run(const std::vector<std::function<void()>>& bodies) {
 }
 
 // A group of two threads over `items` items, blocks of two rows and one as the
-// product kernel takes them.
-template <int L>
-static void products(int items, long lost) {
-    using Keys = ItemKeys<L>;
+// product kernel takes them; items with rotation 0 use no rows.
+template <int L, bool ROT>
+static void products(std::vector<int32_t> rot, long lost) {
+    using Keys = ItemKeys<L, ROT>;
     static uint64_t full[Keys::S];
     static cpx<float> ring[Keys::S * Keys::kRow];
     static char key[64];
@@ -182,21 +185,29 @@ static void products(int items, long lost) {
     reset(lost, Keys::kRowBytes, src);
     int32_t err = 0;
     volatile int abort = 0;
-    Keys k[2] = {{ring, full, &err, &abort, src, 2 * L * Keys::kRowBytes, (uint32_t)items * 2 * L, 0, 0, 0},
-                 {ring, full, &err, &abort, src, 2 * L * Keys::kRowBytes, (uint32_t)items * 2 * L, 0, 0, 1}};
+    const int items = (int)rot.size();
+    std::vector<Keys> k;
+    for (int t = 0; t < 2; ++t)
+        k.push_back(Keys{ring, full, &err, &abort, src, 2 * L * Keys::kRowBytes, rot.data(), 1, items, t, 0, 0, 0, 0, 0});
+    k[0].start();
     k[0].issue();
     const auto block = [&](int rows) {
         for (int u = 1; u >= 0; --u)
             for (int b = 0; b < rows; ++b) k[u].wait(k[u].used + b);
         for (int u = 0; u < 2; ++u) k[u].release(rows, 1);
     };
-    for (int it = 0; it < items; ++it)
+    std::vector<long> want;
+    for (int it = 0; it < items; ++it) {
+        if (ROT && rot[it] == 0) continue;
+        for (int r = 0; r < 2 * L; ++r) want.push_back(2L * L * it + r);
         for (int jp = 0; jp < 2; ++jp) {
             block(2);
             if (L == 3) block(1);
         }
+    }
     k[0].drain();
-    finish(lost, (long)items * 2 * L, err);
+    if (lost < 0 && g_rows != want) fault("rows of the items that use them, in order");
+    finish(lost, (long)want.size(), err);
 }
 
 static const int kS = 4, kL = 3;
@@ -323,8 +334,12 @@ static void pair(long lost, int steps) {
 int main(int, char** argv) {
     const std::string what = argv[1];
     const long lost = std::atol(argv[2]);
-    if (what == "products2") products<2>(3, lost);
-    else if (what == "products3") products<3>(3, lost);
+    if (what == "products2") products<2, false>({0, 0, 0}, lost);
+    else if (what == "products3") products<3, false>({0, 0, 0}, lost);
+    else if (what == "rotations2") products<2, true>({0, 7, 0, 0, 2047, 1, 0}, lost);  // items 1, 4, 5: rows 4, 16, 20 on
+    else if (what == "rotations3") products<3, true>({5, 0, 1, 0}, lost);               // items 0, 2: rows 0, 12 on
+    else if (what == "no_rotation") products<3, true>({0, 0, 0, 0, 0}, lost);
+    else if (what == "no_items") products<3, true>({}, lost);
     else if (what == "ring") ring<false>(lost, false, 3);
     else if (what == "producer_warp") ring<true>(lost, true, 3);
     else if (what == "lane_pairs") polled(lost, 3);

@@ -67,3 +67,28 @@ def test_noiseless_constants_cost_no_steps(pkg, torch_cuda, count, share):
         assert _bootstrap_us(torch, e, 0, zero) < share * _bootstrap_us(torch, e, 0, x)
     finally:
         e.close()
+
+
+def test_rotation_by_nothing_reads_no_key(pkg, torch_cuda):
+    """MuxRotate items with rotation 0 are copies of 8 KB: their 96 KB of key
+    rows stay where they are."""
+    torch = torch_cuda
+    e = pkg.Engine(pkg.default_params())
+    try:
+        count, sp = 3000, torch.cuda.current_stream().cuda_stream
+        keys = torch.empty(count, e.tgsw_fft_bytes("split_fp32"), device="cuda", dtype=torch.uint8)
+        e.tgsw_to_fft(_uniform(torch, count, e.params.tgsw_words()), keys, count, "split_fp32", stream=sp)
+        acc = _uniform(torch, count, 2048)
+        out = torch.empty_like(acc)
+
+        def us(a):
+            return _median_us(torch, lambda: e.tfhe_MuxRotate_FFT(out, acc, keys, a, count, "split_fp32", stream=sp),
+                              calls=20)
+
+        a = torch.randint(1, 2048, (count,), device="cuda", dtype=torch.int32)
+        assert us(torch.zeros_like(a)) < 0.4 * us(a)
+        e.tfhe_MuxRotate_FFT(out, acc, keys, torch.zeros_like(a), count, "split_fp32", stream=sp)
+        torch.cuda.synchronize()
+        assert torch.equal(out, acc)
+    finally:
+        e.close()

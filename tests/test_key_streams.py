@@ -32,6 +32,14 @@ def test_product_stream_ends_by_itself(model, stream, rows):
         assert model(stream, lost) == [], lost
 
 
+# rows only of the items that rotate: zeros first, last, in a row; none; no items
+@pytest.mark.parametrize("stream,rows", [("rotations2", [4, 7, 16, 18, 22, 23]), ("rotations3", [0, 3, 12, 16, 17]),
+                                         ("no_rotation", []), ("no_items", [])])
+def test_product_stream_copies_what_is_used(model, stream, rows):
+    for lost in [-1] + rows:
+        assert model(stream, lost) == [], lost
+
+
 # shared rings: streamed in line, by a producer warp, for lane pairs, for two halves
 @pytest.mark.parametrize("stream", ["ring", "producer_warp", "lane_pairs", "pair"])
 def test_ring_ends_by_itself(model, stream):
