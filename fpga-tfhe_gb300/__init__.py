@@ -568,8 +568,9 @@ class Engine:
         return self.lib.tfhe_gpu_selftest_timeout(self.ctx, self._form(form), int(count))
 
     def selftest_timeout_in(self, part, count):
-        """The same for another part of the engine: "key_switch"."""
-        return self.lib.tfhe_gpu_selftest_timeout_in(self.ctx, {"key_switch": 1}[part], int(count))
+        """The same for another part of the engine: "key_switch" or "product"
+        (split-FP32 external products)."""
+        return self.lib.tfhe_gpu_selftest_timeout_in(self.ctx, {"key_switch": 1, "product": 2}[part], int(count))
 
     def autotune(self, form, count):
         """Time the launch shapes on `count` ciphertexts; keeps and returns

@@ -714,10 +714,7 @@ __global__ void __launch_bounds__(64 * ProductPlan<L>::kGroups, 1)
         a_next = a.bara[first];
         asm volatile("prefetch.global.L1 [%0];" ::"l"(a.acc_in + (size_t)first * 2 * kN + 32 * t));
     }
-    if (t == 0) {  // the first rows travel while the tables load
-        keys.start();
-        keys.issue();
-    }
+    if (t == 0) keys.start(a.stall_keys);  // the first rows travel while the tables load
     load_hot_tables<float>(tables, T);
     __syncthreads();
     if (items == 0) return;

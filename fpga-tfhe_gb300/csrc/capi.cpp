@@ -938,18 +938,31 @@ tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form,
 
 tfhe_gpu_status tfhe_gpu_selftest_timeout_in(tfhe_gpu_ctx* ctx, int32_t part, int32_t count) {
     CHECK_CTX(ctx);
-    if (count <= 0 || part != TFHE_GPU_PART_KEY_SWITCH) return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
+    if (count <= 0 || (part != TFHE_GPU_PART_KEY_SWITCH && part != TFHE_GPU_PART_PRODUCT))
+        return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
+    if (part == TFHE_GPU_PART_PRODUCT) RET(need_bk(ctx, TFHE_GPU_SPLIT_FP32));
+    else if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
     RET(check_device_status(ctx));  // start from a clean status word
-    const int n = ctx->P.n, nk = ctx->P.k * ctx->P.N;
+    const size_t in_words = (part == TFHE_GPU_PART_PRODUCT ? 2 : 1) * (size_t)ctx->P.k * ctx->P.N + 1;
     cudaStream_t st = ctx->stream;
-    void *u = nullptr, *out = nullptr;
-    if (!ctx->has_ks()) return fail(ctx, TFHE_GPU_NO_KEY, "key-switching key not uploaded");
-    RET(ensure_scratch(ctx, 1, (size_t)count * (nk + 1) * sizeof(int32_t), &u));
-    RET(ensure_scratch(ctx, 0, (size_t)count * (n + 1) * sizeof(int32_t), &out));
-    CK(ctx, cudaMemsetAsync(u, 0, (size_t)count * (nk + 1) * sizeof(int32_t), st));
-    KsTable ks = ctx->ks_table();
-    ks.stall = true;
-    CK(ctx, launch_keyswitch(ctx->dp, ks, (const int32_t*)u, (int32_t*)out, count, st));
+    void *in = nullptr, *out = nullptr;
+    RET(ensure_scratch(ctx, 1, count * in_words * sizeof(int32_t), &in));
+    CK(ctx, cudaMemsetAsync(in, 0, count * in_words * sizeof(int32_t), st));
+    if (part == TFHE_GPU_PART_PRODUCT) {
+        EpArgs a{};
+        a.err = ctx->d_err;
+        a.acc_in = (const int32_t*)in;
+        a.acc_out = (int32_t*)in;
+        a.gsw = ctx->d_bk[kFormSplitFp32];
+        a.count = count;
+        a.stall_keys = 1;
+        CK(ctx, launch_external_product(ctx->dp, kFormSplitFp32, kEpPlain, ctx->tables, a, 0, st));
+    } else {
+        RET(ensure_scratch(ctx, 0, (size_t)count * (ctx->P.n + 1) * sizeof(int32_t), &out));
+        KsTable ks = ctx->ks_table();
+        ks.stall = true;
+        CK(ctx, launch_keyswitch(ctx->dp, ks, (const int32_t*)in, (int32_t*)out, count, st));
+    }
     CK(ctx, cudaStreamSynchronize(st));
     return check_device_status(ctx);
 }

@@ -39,11 +39,18 @@ struct ItemKeys {
     // thread 0: the row to issue, and the rotation of the item after its own
     int item, row, ahead;
 
-    // thread 0, once: the first item
-    __device__ __forceinline__ void start() {
+    // thread 0, once: the first rows.  stall: self-test of the waits, the slots
+    // are armed and no copy is started.
+    __device__ __forceinline__ void start(bool stall) {
+        if (stall) {
+            for (; items > 0 && next < S; ++next) mbar_arrive_expect_tx(&full[next], (uint32_t)kRowBytes);
+            item = items;
+            return;
+        }
         item = -1;
         if (ROT && items > 0) ahead = rot[0];
         next_item();
+        issue();
     }
     __device__ __forceinline__ void next_item() {
         row = 0;

@@ -189,8 +189,7 @@ static void products(std::vector<int32_t> rot, long lost) {
     std::vector<Keys> k;
     for (int t = 0; t < 2; ++t)
         k.push_back(Keys{ring, full, &err, &abort, src, 2 * L * Keys::kRowBytes, rot.data(), 1, items, t, 0, 0, 0, 0, 0});
-    k[0].start();
-    k[0].issue();
+    k[0].start(false);
     const auto block = [&](int rows) {
         for (int u = 1; u >= 0; --u)
             for (int b = 0; b < rows; ++b) k[u].wait(k[u].used + b);

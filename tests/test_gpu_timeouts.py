@@ -70,3 +70,32 @@ def test_one_per_cta_rotation_timeout(pkg, torch_cuda, params, shape, count):
         _timeout_then(lambda: e.selftest_timeout("split_fp32", count), check)
     finally:
         e.close()
+
+
+# one group; one a group in every SM; the second of two items a group
+@pytest.mark.parametrize("params,count", [("default", 1), ("stress", 608), ("default", 1000)])
+def test_product_timeout(pkg, torch_cuda, params, count):
+    torch = torch_cuda
+    e = pkg.Engine(pkg.default_params() if params == "default" else pkg.stress_params())
+    try:
+        e.gate_keyset([9], forms=("split_fp32",), want_bk=False)
+        sp = torch.cuda.current_stream().cuda_stream
+        tgsw = torch.randint(-2 ** 31, 2 ** 31, (count, e.params.tgsw_words()), device="cuda", dtype=torch.int32)
+        keys = torch.empty(count, e.tgsw_fft_bytes("split_fp32"), device="cuda", dtype=torch.uint8)
+        e.tgsw_to_fft(tgsw, keys, count, "split_fp32", stream=sp)
+        acc = torch.randint(-2 ** 31, 2 ** 31, (count, 2048), device="cuda", dtype=torch.int32)
+        out = [acc.clone(), acc.clone()]
+
+        def product(k):
+            e.tGswFFTExternMulToTLwe(out[k], keys, count, "split_fp32", stream=sp)
+            torch.cuda.synchronize()
+            e.synchronize()
+
+        def check():
+            product(1)
+            assert torch.equal(out[0], out[1])
+
+        product(0)
+        _timeout_then(lambda: e.selftest_timeout_in("product", count), check)
+    finally:
+        e.close()
