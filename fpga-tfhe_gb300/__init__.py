@@ -568,9 +568,11 @@ class Engine:
         return self.lib.tfhe_gpu_selftest_timeout(self.ctx, self._form(form), int(count))
 
     def selftest_timeout_in(self, part, count):
-        """The same for another part of the engine: "key_switch" or "product"
-        (split-FP32 external products)."""
-        return self.lib.tfhe_gpu_selftest_timeout_in(self.ctx, {"key_switch": 1, "product": 2}[part], int(count))
+        """The same for another part of the engine: "key_switch", "product"
+        (split-FP32 external products) or "cluster_fp64" (stores between the
+        SMs of a cluster)."""
+        parts = {"key_switch": 1, "product": 2, "cluster_fp64": 3}
+        return self.lib.tfhe_gpu_selftest_timeout_in(self.ctx, parts[part], int(count))
 
     def autotune(self, form, count):
         """Time the launch shapes on `count` ciphertexts; keeps and returns

@@ -134,6 +134,14 @@ __device__ __forceinline__ bool mbar_wait_cluster_bounded(uint64_t* bar, uint32_
     return true;
 }
 
+// A kernel that ends after a wait gave up cannot count what it has sent to
+// other CTAs any more: 100 us, a hundred times what such a store takes.
+__device__ __forceinline__ void let_stores_land() {
+    const uint64_t t0 = global_ns();
+    while (global_ns() - t0 < 100000) {
+    }
+}
+
 // Order this thread's shared-memory writes before later reads of the async
 // proxy (bulk copies, matrix instructions).
 __device__ __forceinline__ void fence_proxy_async() {

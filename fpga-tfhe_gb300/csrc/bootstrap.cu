@@ -1774,7 +1774,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
     if (threadIdx.x == 0) {
         mbar_init(&dbar[0], 1);
         mbar_init(&dbar[1], 1);
-        *abort = 0;
+        *abort = a.stall_peers && r == 1;  // self-test: this CTA sends nothing
         fence_mbar_init();
     }
     cluster.sync();  // both CTAs' barriers initialised before any push
@@ -1800,9 +1800,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
         const int ai = bara ? rot_next : mod_switch_2n(rot_next);
         if (i + 1 < n) rot_next = rot[i + 1];
         if (ai == 0) continue;  // tfhe_blindRotate_FFT.cpp:114 (uniform over the cluster)
+        const int stop = *abort;  // the same for the whole CTA: set only between a step's two barriers
         const int buf = (int)(k & 1);
         // this step's incoming digits: one arrival and l x 8 KB of stores
-        if (threadIdx.x == 0) mbar_arrive_expect_tx(&dbar[buf], (uint32_t)(L * kHalf * sizeof(cpx<double>)));
+        if (threadIdx.x == 0 && !stop)
+            mbar_arrive_expect_tx(&dbar[buf], (uint32_t)(L * kHalf * sizeof(cpx<double>)));
         const cpx<double>* step_keys = gsw + (size_t)i * step_elems;
         if (i + 1 < n && threadIdx.x < kRows)  // the next step's rows into L2
             bulk_prefetch_l2(step_keys + step_elems + (size_t)threadIdx.x * kRowElems + r * kHalf,
@@ -1827,6 +1829,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
             v[q] = digit_pair<double>(u0, u1, decal, mask, halfBg);
         }
         fft512_forward_ip1(v, sc.b0, tw, ix, t, bar_id);
+        if (stop) break;  // nothing is armed or sent after a wait has given up
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int e = (lev * 8 + q) * 64 + t;
@@ -1882,6 +1885,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 * L, 1)
             dst[kN] = acc[0];
         }
     }
+    if (*abort) let_stores_land();
     cluster.sync();  // no CTA leaves while its peer could still address its shared memory
 }
 
@@ -2026,7 +2030,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
         mbar_init(bar_acc, 1);
         mbar_init(bar_d, 1);
         mbar_init(bar_p, 1);
-        *abort = 0;
+        *abort = a.stall_peers && m == 0;  // self-test: this CTA sends no points
         fence_mbar_init();
     }
     cluster.sync();  // every CTA's barriers initialised before any store
@@ -2040,8 +2044,12 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
     const int32_t* bara = a.bara ? a.bara + (size_t)c * n : nullptr;
     const int32_t* xs = a.x ? a.x + (size_t)c * (n + 1) : nullptr;
     const int32_t* rot = bara ? bara : xs;
+    // after a wait that gave up a thread arms nothing more, and its CTA leaves
+    // the loop at the next barrier
+    bool ok = true;
     const auto wait_for = [&](uint64_t* bar, uint32_t parity) {
         if (!mbar_wait_cluster_bounded(bar, parity, abort)) {
+            ok = false;
             *abort = 1;
             atomicExch(a.err, 3);
         }
@@ -2054,7 +2062,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
         const int ai = bara ? rot_next : mod_switch_2n(rot_next);
         if (i + 1 < n) rot_next = rot[i + 1];
         if (ai == 0) continue;  // tfhe_blindRotate_FFT.cpp:114 (uniform over the cluster)
-        if (u == 0) {
+        if (u == 0 && ok) {
             mbar_arrive_expect_tx(bar_d, kRows * 64 * sizeof(cpx<double>));
             mbar_arrive_expect_tx(bar_p, 2 * 64 * sizeof(cpx<double>));
         }
@@ -2069,7 +2077,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
         }
         if (forward) {
             if (k > 0) wait_for(bar_acc, (k - 1) & 1);
-            if (u == 0) mbar_arrive_expect_tx(bar_acc, kN * sizeof(int32_t));
+            if (u == 0 && ok) mbar_arrive_expect_tx(bar_acc, kN * sizeof(int32_t));
             __syncwarp();
             const int t = u & 63, hp = u >> 6;
             cpx<double> w[4], y[4];
@@ -2104,12 +2112,14 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
             o0[mj * 72 + 9 * mt + mq] = o;
         }
         __syncthreads();
+        const int stop = *abort;  // the same for the whole CTA: not set between these two barriers
         cpx<double> v[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = o0[wj * 72 + 9 * wt + q];
         // pass C' of butterfly wt, output wq, times pass B''s twiddle
         o1[wj * 72 + 9 * wt + wq] = cmulc_any(dft8_by_warp<-1>(v, warp, minus), tw.b[wt * 8 + wq]);
         __syncthreads();
+        if (stop) break;
         // pass B' of butterfly j = wt (positions j + 8r), output wq, times pass A''s twiddle
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = o1[wj * 72 + 9 * q + wt];
@@ -2160,6 +2170,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
         }
     }
     if (forward && k > 0) wait_for(bar_acc, (k - 1) & 1);  // the last coefficients landed
+    if (*abort) let_stores_land();
     cluster.sync();  // no CTA leaves while another could still address its shared memory
 }
 

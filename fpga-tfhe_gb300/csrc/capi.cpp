@@ -910,8 +910,7 @@ tfhe_gpu_status tfhe_gpu_autotune(tfhe_gpu_ctx* ctx, tfhe_gpu_form form, int32_t
     return TFHE_GPU_OK;
 }
 
-tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form, int32_t count) {
-    CHECK_CTX(ctx);
+static tfhe_gpu_status stalled_rotation(tfhe_gpu_ctx* ctx, tfhe_gpu_form form, int32_t count, bool peers) {
     if (count <= 0) return fail(ctx, TFHE_GPU_BAD_PARAM, "count");
     RET(need_bk(ctx, form));
     RET(check_device_status(ctx));  // start from a clean status word
@@ -929,15 +928,22 @@ tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form,
     a.lwe_out = (int32_t*)u;
     a.gsw = ctx->d_bk[form];
     a.count = count;
-    a.stall_keys = 1;
+    a.stall_keys = !peers;
+    a.stall_peers = peers;
     CK(ctx, launch_external_product(ctx->dp, (Form)form, kEpBlindRotate, ctx->tables, a,
                                     ctx->groups_per_cta[form], st));
     CK(ctx, cudaStreamSynchronize(st));
     return check_device_status(ctx);
 }
 
+tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form, int32_t count) {
+    CHECK_CTX(ctx);
+    return stalled_rotation(ctx, form, count, false);
+}
+
 tfhe_gpu_status tfhe_gpu_selftest_timeout_in(tfhe_gpu_ctx* ctx, int32_t part, int32_t count) {
     CHECK_CTX(ctx);
+    if (part == TFHE_GPU_PART_CLUSTER_FP64) return stalled_rotation(ctx, TFHE_GPU_FP64, count, true);
     if (count <= 0 || (part != TFHE_GPU_PART_KEY_SWITCH && part != TFHE_GPU_PART_PRODUCT))
         return fail(ctx, TFHE_GPU_BAD_PARAM, "args");
     if (part == TFHE_GPU_PART_PRODUCT) RET(need_bk(ctx, TFHE_GPU_SPLIT_FP32));

@@ -84,6 +84,9 @@ struct EpArgs {
     // copy key rows into shared memory start none of the copies, so every wait
     // for them runs out
     int32_t stall_keys;
+    // the same (tfhe_gpu_selftest_timeout_in) for the FP64 kernels over clusters:
+    // one CTA of each sends the others nothing
+    int32_t stall_peers;
 };
 
 cudaError_t launch_external_product(const DevParams& P, Form f, EpMode mode,

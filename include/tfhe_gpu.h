@@ -337,9 +337,13 @@ tfhe_gpu_status tfhe_gpu_selftest_timeout(tfhe_gpu_ctx* ctx, tfhe_gpu_form form,
  *   TFHE_GPU_PART_KEY_SWITCH: a key switch whose table stream ends after its
  *     first stage (TFHE_GPU_OK for ks_t other than 8, which has no waits);
  *   TFHE_GPU_PART_PRODUCT: split-FP32 external products whose copies of key
- *     rows are never started (the key is the context's bootstrapping key). */
+ *     rows are never started (the key is the context's bootstrapping key);
+ *   TFHE_GPU_PART_CLUSTER_FP64: an FP64 blind rotation with the current launch
+ *     shape in which one SM of each cluster sends the others nothing
+ *     (TFHE_GPU_OK for shapes without clusters). */
 #define TFHE_GPU_PART_KEY_SWITCH 1
 #define TFHE_GPU_PART_PRODUCT 2
+#define TFHE_GPU_PART_CLUSTER_FP64 3
 tfhe_gpu_status tfhe_gpu_selftest_timeout_in(tfhe_gpu_ctx* ctx, int32_t part, int32_t count);
 
 /* Measured FP32 FMA-pipe peak of `device` in TFLOP/s (and the probe's

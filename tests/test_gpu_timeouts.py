@@ -99,3 +99,30 @@ def test_product_timeout(pkg, torch_cuda, params, count):
         _timeout_then(lambda: e.selftest_timeout_in("product", count), check)
     finally:
         e.close()
+
+
+# FP64 over two SMs and over eight
+@pytest.mark.parametrize("params,shape,count", [("default", 16, 2), ("stress", 0, 60), ("default", 0, 1),
+                                                ("stress", 0, 30)])
+def test_cluster_timeout(pkg, torch_cuda, params, shape, count):
+    torch, form = torch_cuda, "fp64"
+    e = pkg.Engine(pkg.default_params() if params == "default" else pkg.stress_params())
+    try:
+        e.gate_keyset([9], forms=(form,), want_bk=False)
+        x = torch.randint(-2 ** 31, 2 ** 31, (count, e.params.n + 1), device="cuda", dtype=torch.int32)
+        out = torch.empty((2, count, 1025), device="cuda", dtype=torch.int32)
+        e.set_groups_per_cta(form, shape)
+
+        def bootstrap(k):
+            e.tfhe_bootstrap_woKS_FFT(out[k], x, 1 << 29, count, form, stream=torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            e.synchronize()
+
+        def check():
+            bootstrap(1)
+            assert torch.equal(out[0], out[1])
+
+        bootstrap(0)
+        _timeout_then(lambda: e.selftest_timeout_in("cluster_fp64", count), check)
+    finally:
+        e.close()
