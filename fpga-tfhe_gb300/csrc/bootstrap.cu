@@ -1954,7 +1954,7 @@ __device__ __forceinline__ void forward_parity(cpx<double> (&w)[4], cpx<double> 
     cpx<double> v[8];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        if (4 * H + k) w[k] = cmul_const(w[k], twist_c<double>(4 * H + k));
+        if (4 * H + k) w[k] = cmul_alt(w[k], twist_c<double>(4 * H + k));
         x0[spad(t + 64 * (4 * H + k))] = w[k];
     }
     parity_sync();
@@ -1962,7 +1962,7 @@ __device__ __forceinline__ void forward_parity(cpx<double> (&w)[4], cpx<double> 
     for (int q = 0; q < 8; ++q) v[q] = x0[spad(t + 64 * q)];
     dft8_parity<1, H>(v, y);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) x1[spad(t + 64 * (2 * k + H))] = cmul_table(y[k], tw.a[(2 * k + H) * 64 + t]);
+    for (int k = 0; k < 4; ++k) x1[spad(t + 64 * (2 * k + H))] = cmul(y[k], tw.a[(2 * k + H) * 64 + t]);
     parity_sync();
     const int b = t >> 3, j = t & 7;
 #pragma unroll
@@ -1970,7 +1970,7 @@ __device__ __forceinline__ void forward_parity(cpx<double> (&w)[4], cpx<double> 
     dft8_parity<1, H>(v, y);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        if (2 * k + H) y[k] = cmul_table(y[k], tw.b[(2 * k + H) * 8 + j]);
+        if (2 * k + H) y[k] = cmul(y[k], tw.b[(2 * k + H) * 8 + j]);
         x0[spad(64 * b + j + 8 * (2 * k + H))] = y[k];
     }
     parity_sync();
@@ -2106,8 +2106,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
             cpx<double> o = {0.0, 0.0};
 #pragma unroll
             for (int p = 0; p < kRows; ++p) {
-                const cpx<double> z = cmul_table(din[p * 64 + mq * 8 + mt], cpx<double>{kk[p].x, kk[p].y});
-                o = {__dadd_rn(o.x, z.x), __dadd_rn(o.y, z.y)};
+                o = cmac(o, din[p * 64 + mq * 8 + mt], cpx<double>{kk[p].x, kk[p].y});
             }
             o0[mj * 72 + 9 * mt + mq] = o;
         }
@@ -2117,14 +2116,14 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = o0[wj * 72 + 9 * wt + q];
         // pass C' of butterfly wt, output wq, times pass B''s twiddle
-        o1[wj * 72 + 9 * wt + wq] = cmulc_any(dft8_by_warp<-1>(v, warp, minus), tw.b[wt * 8 + wq]);
+        o1[wj * 72 + 9 * wt + wq] = cmulc(dft8_by_warp<-1>(v, warp, minus), tw.b[wt * 8 + wq]);
         __syncthreads();
         if (stop) break;
         // pass B' of butterfly j = wt (positions j + 8r), output wq, times pass A''s twiddle
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = o1[wj * 72 + 9 * q + wt];
         {
-            const cpx<double> z = cmulc_any(dft8_by_warp<-1>(v, warp, minus), tw.a[m * 64 + wt + 8 * wq]);
+            const cpx<double> z = cmulc(dft8_by_warp<-1>(v, warp, minus), tw.a[m * 64 + wt + 8 * wq]);
             st_async_d2(cluster_map(smem_u32(pin), (uint32_t)wq) +
                             (uint32_t)(((wj * 8 + m) * 8 + wt) * sizeof(cpx<double>)),
                         z.x, z.y, cluster_map(smem_u32(bar_p), (uint32_t)wq));
@@ -2139,7 +2138,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(Cluster8F64Plan<L>::
 #pragma unroll
             for (int q = 1; q < 8; ++q)
                 if (wq == q) un = twist_c<double>(q);
-            z = cmulc_any(z, un);
+            z = cmulc(z, un);
             own0 += trunc_div512(z.x);
             own1 += trunc_div512(z.y);
             const int x = 8 * m + wt + 64 * wq;
@@ -2524,7 +2523,7 @@ __device__ __forceinline__ void twisted_forward64(const double* coef, cpx<double
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int x0 = t + 64 * r;
-        v[r] = cmul(cpx<double>{coef[x0], coef[x0 + kHalf]}, psi[x0]);
+        v[r] = cmul_alt(cpx<double>{coef[x0], coef[x0 + kHalf]}, psi[x0]);
     }
     fft512_forward(v, s, tw, t, bar);
 }

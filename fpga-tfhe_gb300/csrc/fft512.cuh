@@ -57,6 +57,48 @@ __device__ __forceinline__ cpx<R> cmac(cpx<R> acc, cpx<R> a, cpx<R> w) {
     return cadd(acc, cmul(a, w));
 }
 
+// ---- FP64: every rounding spelt out --------------------------------------
+// Which product of a sum of two is fused into the addition would otherwise be
+// the compiler's choice, and could differ between two kernels that have to
+// give the same ciphertext bit for bit.  cmul_alt fuses the other product of
+// the imaginary part: the blind rotations and products use it for the twist's
+// constants, the transforms of keys and polynomials (fft512_forward) throughout.
+__device__ __forceinline__ cpx<double> cadd(cpx<double> a, cpx<double> b) {
+    return {__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)};
+}
+__device__ __forceinline__ cpx<double> csub(cpx<double> a, cpx<double> b) {
+    return {__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y)};
+}
+__device__ __forceinline__ cpx<double> cmul(cpx<double> a, cpx<double> w) {
+    return {__fma_rn(a.x, w.x, -__dmul_rn(a.y, w.y)), __fma_rn(a.x, w.y, __dmul_rn(a.y, w.x))};
+}
+__device__ __forceinline__ cpx<double> cmul_alt(cpx<double> a, cpx<double> c) {
+    return {__fma_rn(a.x, c.x, -__dmul_rn(a.y, c.y)), __fma_rn(a.y, c.x, __dmul_rn(a.x, c.y))};
+}
+__device__ __forceinline__ cpx<double> cmulc(cpx<double> a, cpx<double> w) {
+    return {__fma_rn(a.x, w.x, __dmul_rn(a.y, w.y)), __fma_rn(a.y, w.x, -__dmul_rn(a.x, w.y))};
+}
+__device__ __forceinline__ cpx<double> cmac(cpx<double> acc, cpx<double> a, cpx<double> w) {
+    return cadd(acc, cmul(a, w));
+}
+// (a + b) h and (a - b) h, b's product rounded first
+__device__ __forceinline__ cpx<double> scaled_sum(cpx<double> a, cpx<double> b, double h) {
+    return {__fma_rn(a.x, h, __dmul_rn(b.x, h)), __fma_rn(a.y, h, __dmul_rn(b.y, h))};
+}
+__device__ __forceinline__ cpx<double> scaled_diff(cpx<double> a, cpx<double> b, double h) {
+    return {__fma_rn(a.x, h, -__dmul_rn(b.x, h)), __fma_rn(a.y, h, -__dmul_rn(b.y, h))};
+}
+constexpr double kSqrtHalf = 0.70710678118654752440084436210485;
+// a times (1 + S i) and (-1 + S i), S = +-1
+template <int S>
+__device__ __forceinline__ cpx<double> times_1i(cpx<double> a) {
+    return {__dadd_rn(a.x, -S * a.y), __dadd_rn(a.y, S * a.x)};
+}
+template <int S>
+__device__ __forceinline__ cpx<double> times_m1i(cpx<double> a) {
+    return {__dadd_rn(-a.x, -S * a.y), __dadd_rn(S * a.x, -a.y)};
+}
+
 // ---- FP32: packed pair arithmetic ---------------------------------------
 // A complex float is one 64-bit register pair and add/mul/fma.f32x2 (sm_100
 // and later) work on both halves in one instruction, so complex adds take
@@ -86,6 +128,7 @@ __device__ __forceinline__ cpx<float> cmul(cpx<float> a, cpx<float> w) {
 __device__ __forceinline__ cpx<float> cmulc(cpx<float> a, cpx<float> w) {
     return unpk(__ffma2_rn(times_minus_i(a), bc(w.y), __fmul2_rn(pk(a), bc(w.x))));
 }
+__device__ __forceinline__ cpx<float> cmul_alt(cpx<float> a, cpx<float> c) { return cmul(a, c); }
 __device__ __forceinline__ cpx<float> cmac(cpx<float> acc, cpx<float> a, cpx<float> w) {
     return unpk(__ffma2_rn(times_i(a), bc(w.y), __ffma2_rn(pk(a), bc(w.x), pk(acc))));
 }
@@ -153,31 +196,23 @@ __device__ __forceinline__ void dft8(cpx<R> (&v)[8]) {
     if constexpr (sizeof(R) == 4) {
         dft8_f32<S>(v);
     } else {
-        const R h = (R)0.70710678118654752440084436210485;
         cpx<R> b[8];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             b[r] = cadd(v[r], v[r + 4]);
             b[r + 4] = csub(v[r], v[r + 4]);
         }
-        {  // b5 *= w = (1 + S i) h
-            const R x = b[5].x, y = b[5].y;
-            b[5] = {(x - S * y) * h, (y + S * x) * h};
-        }
-        {  // b6 *= w^2 = S i
-            const R x = b[6].x, y = b[6].y;
-            b[6] = {-S * y, S * x};
-        }
-        {  // b7 *= w^3 = (-1 + S i) h
-            const R x = b[7].x, y = b[7].y;
-            b[7] = {(-x - S * y) * h, (S * x - y) * h};
-        }
+        // b5 (w = (1 + S i) h) and b7 (w^3 = (-1 + S i) h) without their h, b6 w^2 = S i b6
+        b[5] = times_1i<S>(b[5]);
+        b[6] = {-S * b[6].y, S * b[6].x};
+        b[7] = times_m1i<S>(b[7]);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const cpx<R> c0 = b[4 * half + 0], c1 = b[4 * half + 1];
             const cpx<R> c2 = b[4 * half + 2], c3 = b[4 * half + 3];
-            const cpx<R> e0 = cadd(c0, c2), e1 = csub(c0, c2), e2 = cadd(c1, c3);
-            const cpx<R> d = csub(c1, c3);
+            const cpx<R> e0 = cadd(c0, c2), e1 = csub(c0, c2);
+            const cpx<R> e2 = half ? scaled_sum(c1, c3, kSqrtHalf) : cadd(c1, c3);
+            const cpx<R> d = half ? scaled_diff(c1, c3, kSqrtHalf) : csub(c1, c3);
             const cpx<R> e3 = {-S * d.y, S * d.x};
             v[half + 0] = cadd(e0, e2);
             v[half + 2] = cadd(e1, e3);
@@ -187,55 +222,38 @@ __device__ __forceinline__ void dft8(cpx<R> (&v)[8]) {
     }
 }
 
-// FP64 complex products with their fused operations spelt out.  Which product
-// of a sum of two is fused is otherwise the compiler's choice, which differs
-// between kernels; these are the choices it makes in the whole-transform FP64
-// kernels (fft512_forward_ip1 and so on), found by emulating their outputs:
-// a w for a table value w, a c for a constant c, a conj(w).
-__device__ __forceinline__ cpx<double> cmul_table(cpx<double> a, cpx<double> w) {
-    return {__fma_rn(a.x, w.x, -__dmul_rn(a.y, w.y)), __fma_rn(a.x, w.y, __dmul_rn(a.y, w.x))};
-}
-__device__ __forceinline__ cpx<double> cmul_const(cpx<double> a, cpx<double> c) {
-    return {__fma_rn(a.x, c.x, -__dmul_rn(a.y, c.y)), __fma_rn(a.y, c.x, __dmul_rn(a.x, c.y))};
-}
-__device__ __forceinline__ cpx<double> cmulc_any(cpx<double> a, cpx<double> w) {
-    return {__fma_rn(a.x, w.x, __dmul_rn(a.y, w.y)), __fma_rn(a.y, w.x, -__dmul_rn(a.x, w.y))};
-}
-
 // Parts of dft8 for butterflies shared by several threads, with its
 // operations on the same operands (so the same bits): the outputs of one
 // parity (q = 2k + H into y[k]), and the two outputs q = 2(C & 1) + (C >> 1)
 // and q + 4, of which `minus` picks the second.
-template <int S, int H, typename R>
-__device__ __forceinline__ void dft8_quad(const cpx<R> (&v)[8], cpx<R> (&b)[4]) {
+template <int S, int H>
+__device__ __forceinline__ void dft8_quad(const cpx<double> (&v)[8], cpx<double> (&b)[4]) {
     if constexpr (H == 0) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) b[r] = cadd(v[r], v[r + 4]);
-    } else {
-        const R h = (R)0.70710678118654752440084436210485;
+    } else {  // b1 and b3 without their factor h
 #pragma unroll
         for (int r = 0; r < 4; ++r) b[r] = csub(v[r], v[r + 4]);
-        {
-            const R x = b[1].x, y = b[1].y;
-            b[1] = {(x - S * y) * h, (y + S * x) * h};
-        }
-        {
-            const R x = b[2].x, y = b[2].y;
-            b[2] = {-S * y, S * x};
-        }
-        {
-            const R x = b[3].x, y = b[3].y;
-            b[3] = {(-x - S * y) * h, (S * x - y) * h};
-        }
+        b[1] = times_1i<S>(b[1]);
+        b[2] = {-S * b[2].y, S * b[2].x};
+        b[3] = times_m1i<S>(b[3]);
     }
 }
-template <int S, int H, typename R>
-__device__ __forceinline__ void dft8_parity(const cpx<R> (&v)[8], cpx<R> (&y)[4]) {
-    cpx<R> b[4];
+template <int H>
+__device__ __forceinline__ cpx<double> quad_sum(cpx<double> b1, cpx<double> b3) {
+    return H ? scaled_sum(b1, b3, kSqrtHalf) : cadd(b1, b3);
+}
+template <int H>
+__device__ __forceinline__ cpx<double> quad_diff(cpx<double> b1, cpx<double> b3) {
+    return H ? scaled_diff(b1, b3, kSqrtHalf) : csub(b1, b3);
+}
+template <int S, int H>
+__device__ __forceinline__ void dft8_parity(const cpx<double> (&v)[8], cpx<double> (&y)[4]) {
+    cpx<double> b[4];
     dft8_quad<S, H>(v, b);
-    const cpx<R> e0 = cadd(b[0], b[2]), e1 = csub(b[0], b[2]), e2 = cadd(b[1], b[3]);
-    const cpx<R> d = csub(b[1], b[3]);
-    const cpx<R> e3 = {-S * d.y, S * d.x};
+    const cpx<double> e0 = cadd(b[0], b[2]), e1 = csub(b[0], b[2]), e2 = quad_sum<H>(b[1], b[3]);
+    const cpx<double> d = quad_diff<H>(b[1], b[3]);
+    const cpx<double> e3 = {-S * d.y, S * d.x};
     y[0] = cadd(e0, e2);
     y[1] = cadd(e1, e3);
     y[2] = csub(e0, e2);
@@ -251,10 +269,10 @@ __device__ __forceinline__ cpx<double> dft8_one(const cpx<double> (&v)[8], bool 
     cpx<double> e, f;
     if constexpr ((C & 1) == 0) {
         e = cadd(b[0], b[2]);
-        f = cadd(b[1], b[3]);
+        f = quad_sum<(C >> 1)>(b[1], b[3]);
     } else {
         e = csub(b[0], b[2]);
-        const cpx<double> d = csub(b[1], b[3]);
+        const cpx<double> d = quad_diff<(C >> 1)>(b[1], b[3]);
         f = {-S * d.y, S * d.x};
     }
     return cadd(e, cpx<double>{flip_sign(f.x, minus), flip_sign(f.y, minus)});
@@ -303,7 +321,7 @@ __device__ __forceinline__ void fft512_forward(cpx<R> (&v)[8], const FftScratch<
     // pass A
     dft8<1>(v);
 #pragma unroll
-    for (int q = 1; q < 8; ++q) v[q] = cmul(v[q], tw.a[q * 64 + t]);
+    for (int q = 1; q < 8; ++q) v[q] = cmul_alt(v[q], tw.a[q * 64 + t]);
 #pragma unroll
     for (int q = 0; q < 8; ++q) s.b0[slot<R>(t + 64 * q)] = v[q];
     group_sync(bar_id);
@@ -313,7 +331,7 @@ __device__ __forceinline__ void fft512_forward(cpx<R> (&v)[8], const FftScratch<
     for (int r = 0; r < 8; ++r) v[r] = s.b0[slot<R>(64 * b + j + 8 * r)];
     dft8<1>(v);
 #pragma unroll
-    for (int q = 1; q < 8; ++q) v[q] = cmul(v[q], tw.b[q * 8 + j]);
+    for (int q = 1; q < 8; ++q) v[q] = cmul_alt(v[q], tw.b[q * 8 + j]);
 #pragma unroll
     for (int q = 0; q < 8; ++q) s.b1[slot<R>(64 * b + j + 8 * q)] = v[q];
     group_sync(bar_id);
@@ -427,7 +445,7 @@ __device__ __forceinline__ void fft512_forward_tw_multi(cpx<R> (&v)[NB][8], cons
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
 #pragma unroll
-        for (int r = 1; r < 8; ++r) v[b][r] = cmul(v[b][r], twist_c<R>(r));
+        for (int r = 1; r < 8; ++r) v[b][r] = cmul_alt(v[b][r], twist_c<R>(r));
         dft8<1>(v[b]);
     }
 #pragma unroll
@@ -548,7 +566,7 @@ __device__ __forceinline__ void fft512_forward_ip(cpx<R> (&v)[NB][8], cpx<R>* co
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
 #pragma unroll
-        for (int r = 1; r < 8; ++r) v[b][r] = cmul(v[b][r], twist_c<R>(r));
+        for (int r = 1; r < 8; ++r) v[b][r] = cmul_alt(v[b][r], twist_c<R>(r));
         dft8<1>(v[b]);
     }
 #pragma unroll
@@ -709,7 +727,7 @@ __device__ __forceinline__ void fft512_forward_duo(cpx<R> (&v)[NB][8], cpx<R>* c
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
 #pragma unroll
-        for (int r = 1; r < 8; ++r) v[b][r] = cmul(v[b][r], twist_c<R>(r));
+        for (int r = 1; r < 8; ++r) v[b][r] = cmul_alt(v[b][r], twist_c<R>(r));
         dft8<1>(v[b]);
     }
 #pragma unroll
