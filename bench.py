@@ -59,10 +59,10 @@ FLOP_PER_BOOTSTRAP = 162.6e6      # FFT-form algorithmic count, default set
 DRAM_KEY_BYTES_PER_LAUNCH = 61.9e6
 # Shared-memory wavefronts per bootstrap of the batched ring kernels (the
 # shared-memory wavefront count of a full ncu capture of each: 1.26 G for a
-# 912-gate wave in lane pairs, summarised in
-# profiles/kernels_lane_pairs_keyswitch_mma_fp64_cluster8.md; 0.74 G for a
-# 448-gate wave of the 4-per-SM kernel, and 1.58 G for the 6-per-SM kernel
-# before the lane pairs, both in
+# 912-gate wave in lane pairs, 0.74 G for 448 gates 3 per CTA and for 448 gates
+# 4 per CTA, summarised in
+# profiles/kernels_lane_pairs_keyswitch_mma_fp64_cluster8.md; 1.58 G for the
+# 6-per-SM kernel before the lane pairs, which nothing launches any more, in
 # profiles/blind_rotate_ring_pairs_batched_keyswitch_batch1360.md).  The
 # shared-memory pipe serves one wavefront per SM clock.
 SMEM_WAVEFRONTS_PER_BOOTSTRAP = {
@@ -1058,10 +1058,8 @@ def main():
             "decrypt_ok": ok,
             "e2e": {"value": e2e_value, "unit": "bootstraps/s",
                     "h2d_bytes_per_step": 2 * lwe_bytes + batch * 4, "d2h_bytes_per_step": lwe_bytes},
-            # eager: combine, the blind rotations, one key switch (two when full
-            # waves leave a remainder of at most 4 per SM)
             "gpu_launches": (graph.kernels if graph is not None
-                             else 1 + br_launches + (2 if batch > 6 * SMS and 0 < batch % (6 * SMS) <= 4 * SMS else 1))
+                             else eager_gate_launches(args.form, eng.get_groups_per_cta(args.form), batch))
             * args.steps,
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak,
@@ -1204,15 +1202,34 @@ def launched_blind_rotations(form, shape, batch, l=3):
             names += [batched(most) + " x %d" % most]
             return names + (low(rest - most) if rest > most else [])
         return names + low(rest, rest > SMS and shape == 0)
-    if form != "fp64" and shape in (9, 10):
+    if form == "fp64":
+        return [{3: "k_external_product<double,1,BlindRotate,3,%d>" % l,
+                 4: "k_blind_rotate_ring<double,1,4,%d,4,inline>" % l,
+                 16: "k_blind_rotate_spread2_f64<%d>" % l}[shape]]
+    if shape in (9, 10):
         return [batched(batch) if shape == 9 else duo % 3]
-    return blind_rotate_kernels(form, shape, batch, l)
+    if shape in (11, 12, 13):
+        return ["k_blind_rotate_pair<float,2,%d,%d,4>" % (shape - 10, l)]
+    if shape in (14, 16):
+        return ["k_blind_rotate_spread%s<%d>" % ("2" if shape == 16 else "", l)]
+    if shape in (1, 2, 4):
+        return ["k_external_product<float,2,BlindRotate,%d,%d>" % (shape, l)]
+    return ["k_blind_rotate_ring<float,2,%d,%d,4,%s>" % (shape, l, "producer-warp" if shape == 5 else "inline")]
+
+
+def eager_gate_launches(form, shape, batch, l=3):
+    """Kernels of one eager gate batch: the combination, the blind rotations and
+    one key switch -- two when the engine switches the full waves' outputs beside
+    the remainder (blind_rotate_tail_start of csrc/bootstrap.cu)."""
+    rest = batch % (6 * SMS)
+    forked = form != "fp64" and shape in (0, 15) and batch > 6 * SMS and 0 < rest <= 4 * SMS
+    return 1 + len(launched_blind_rotations(form, shape, batch, l)) + (2 if forked else 1)
 
 
 def blind_rotate_kernels(form, shape, batch, l=3):
-    """Launch accounting by the shapes' first kernels: which shape a batch's
-    parts fall to, in those names (launched_blind_rotations has the kernels
-    that run them now)."""
+    """Which shape a batch's parts fell to before the lane-pair, spread and
+    eight-SM kernels took ranges over, in the names of that time
+    (launched_blind_rotations has what runs)."""
     if form == "fp64":
         if shape == 16 or (shape == 0 and batch <= SMS):
             return ["k_blind_rotate_spread2_f64<%d>" % l]
