@@ -939,11 +939,11 @@ __global__ void __launch_bounds__(64 * GROUPS + (INLINE ? 0 : 32), 1)
 // nothing.
 //
 // What bounds it: the FP32 pipe and the register file's operand reads
-// together with the latency of 12 warps per SM (FMA pipe 52 %, issue 54 %,
-// shared-memory pipe 64 %).  Against one ciphertext per 64 threads, which was
+// together with the latency of 12 warps per SM (FMA pipe 54 %, issue 55 %,
+// shared-memory pipe 67 %).  Against one ciphertext per 64 threads, which was
 // at 80 % of the shared-memory pipe (key rows and twiddles 1,130 of 2,750
-// wavefronts per ciphertext and step): 6.41 -> 6.23 ms for 912 ciphertexts of
-// the default set, 4.03 -> 3.88 ms for l = 2.  Eight per SM with transforms
+// wavefronts per ciphertext and step): 6.41 -> 6.12 ms for 912 ciphertexts of
+// the default set, 4.03 -> 3.84 ms for l = 2.  Eight per SM with transforms
 // one at a time took 8.5 ms for 1,216; unrolling over the two input
 // polynomials 10.5 ms (the code no longer fits the instruction cache).
 // ----------------------------------------------------------------------
@@ -978,7 +978,7 @@ struct DuoCtx {
 // point come one after another: v[q] is then the same register operand of
 // eight packed FMAs in a row.  A packed FMA with three different register
 // pairs takes 3 clocks (operand reads), with one reused 2.1 to 2.4; this
-// order is 0.11 ms of the 6.23.
+// order is 0.11 ms of a 912-ciphertext wave.
 __device__ __forceinline__ void duo_mac_row(cpx<float> (&out)[2][2][8], const cpx<float> (&v)[8],
                                             const cpx<float>* __restrict__ g, int t) {
     const float4* g4 = reinterpret_cast<const float4*>(g) + t;
@@ -1189,13 +1189,13 @@ __global__ void __launch_bounds__(kDuoThreads * SETS, 1) k_blind_rotate_duo(KPar
 // each input polynomial on their own, then the two sums (for the batch sizes
 // that shape 0 has always run in that order).
 //
-// What bounds it: the shared-memory pipe (about 4,300 wavefronts of a step's
-// 5,200 clocks: the key values written and read 1,536, the transforms'
-// exchanges 1,280, the digits 580) and the chain of a step's phases.
+// What bounds it: the shared-memory pipe (about 3,600 wavefronts of a step's
+// 5,150 clocks: the key values written and read 1,536, the transforms'
+// exchanges 1,280, the digits 580, the accumulator) and the chain of a step's phases.
 // Measured against the form with one transform per 64 threads, the high and
 // the low part in different groups, keys loaded into registers (the loads
 // held the load/store unit for 600 clocks a step) and accumulated by
-// shared-memory atomics: 1.755 -> 1.574 ms for 152 ciphertexts; the twiddles
+// shared-memory atomics: 1.755 -> 1.570 ms for 152 ciphertexts; the twiddles
 // in registers instead of shared memory are 0.054 ms of that.
 // ----------------------------------------------------------------------
 template <int L>
@@ -3006,10 +3006,10 @@ cudaError_t launch_low_latency(const DevParams& P, const Tables& T, const EpArgs
 
 // Automatic shape of a split-FP32 blind rotation over `count` ciphertexts.
 // Measured per launch (default set): a wave of 6 per SM on
-// launch_ring_pairs 6.2 ms, of 4 per SM on launch_ring_batched 4.6 ms (4.2
-// to 4.3 ms up to 3 per SM), whatever the fill of the wave; the cluster kernel 1.12 ms for up to one
-// per two SMs; the spread kernel 1.58 ms at 1 per SM, 3.0 to 3.2 ms for two
-// waves.  So: whole waves of 6 per SM; a remainder of up to 2 per SM on those
+// launch_ring_pairs 6.1 ms, of 4 per SM on launch_ring_batched 4.6 ms (4.2 ms
+// up to 3 per SM), whatever the fill of the wave; the cluster kernel 1.12 ms
+// for up to one per two SMs; the spread kernel 1.57 ms at 1 per SM, 3.0 to 3.1
+// ms for two waves.  So: whole waves of 6 per SM; a remainder of up to 2 per SM on those
 // two (2.7 ms up to 1.5 per SM, where the pair kernel took 3.24 ms for any
 // count of 2 per SM), of up to 4 per SM as one launch_ring_batched wave, of
 // up to 5 as that wave and the rest on the low-latency kernels (5.7 or 6.1
@@ -3048,7 +3048,9 @@ cudaError_t launch_auto_fp32(const DevParams& P, const Tables& T, const EpArgs& 
 // ms to 48, 20.9 ms at 57; the two-SM cluster kernel 20.3 ms for up to one
 // ciphertext per two SMs; the one-per-CTA kernel 29.8 ms a wave of one per SM; the 3-per-CTA kernel with
 // L2-direct key reads 87.0 ms a wave of three per SM (3 waves of the former
-// take 89.3 ms).  So whole waves of three per SM, and a remainder of up to
+// take 89.3 ms).  The rule takes one kernel per remainder (by these times 77 to
+// 91, 153 to 228 and 305 to 380 would end sooner split between two): whole
+// waves of three per SM, and a remainder of up to
 // two per SM on the one-per-CTA kernel, of up to one per two SMs on the
 // two-SM cluster kernel, of up to 48 on the eight-SM one.
 template <int L>
@@ -3217,8 +3219,14 @@ cudaError_t launch_engine64_to_lagrange_ref(const void* eng, double* ref, int np
 }
 
 int blind_rotate_tail_start(Form f, int groups, int count) {
-    // launch_auto_fp32's split: whole 6-per-SM waves, then a remainder of
-    // at most 4 per SM that runs as its own launch on part of the SMs
+    // launch_auto_fp32's whole 6-per-SM waves, when a remainder of at most 4 per
+    // SM follows as its own launches.  The key switch of the full waves beside
+    // it saves what SMs without a CTA of the remainder can take of it (a
+    // key-switch CTA needs an SM's shared memory to itself): 950 gates 7.38 ->
+    // 7.31 ms, 1,300 10.43 -> 10.38, 1,520 10.77 -> 10.75; nothing at 448 over
+    // whole waves (150 of 152 SMs taken: 4,096 gates 28.97 ms either way).  A
+    // remainder of 4 to 5 per SM is not split off: it leaves SMs free only in its
+    // last launch (912 + 760 gates 12.38 ms, with the fork 12.32).
     if (f != kFormSplitFp32 || (groups != 0 && groups != 15)) return 0;
     const int wave = 6 * kSmCount;
     const int full = (count / wave) * wave;

@@ -173,9 +173,9 @@ tfhe_gpu_status run_gates_in(tfhe_gpu_ctx* ctx, const int32_t* gates, int32_t un
         CK(ctx, launch_keyswitch(ctx->dp, ctx->ks_table(), u, out, count, st));
         return TFHE_GPU_OK;
     }
-    // The remainder wave of the blind rotation occupies only part of the
-    // SMs: issue it right after the full waves, and the full waves' key
-    // switch on the side stream, which fills the idle SMs meanwhile.
+    // The remainder of the blind rotation leaves some SMs without a CTA, how
+    // many depends on its count: issue it right after the full waves, and the
+    // full waves' key switch on the side stream, which takes those SMs.
     const int n = ctx->P.n, nk = ctx->P.k * ctx->P.N;
     RET(run_bootstrap_woks(ctx, x, mu, u, split, form, st));
     CK(ctx, cudaEventRecord(ctx->ev_fork, st));

@@ -19,7 +19,7 @@ struct tfhe_gpu_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     // fork/join of a gate batch: the key switch of the full blind-rotation
-    // waves runs on `side` while the remainder wave leaves SMs idle
+    // waves runs on `side` beside the remainder, on the SMs that it leaves free
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     void* d_tables = nullptr;  // transform tables: FP64 copy then FP32 copy

@@ -120,8 +120,9 @@ cudaError_t launch_lagrange_addmul(const double* a, const double* b,
                                    cudaStream_t st);
 
 // Where the automatic split-FP32 blind rotation of `count` ciphertexts
-// starts its remainder launch (one that leaves SMs idle), or 0 when it is a
-// single launch or another shape is set.
+// starts its remainder, for a key switch of the full waves beside it; 0 when
+// there are no full waves, no remainder or one of more than 4 per SM, or
+// another shape is set.
 int blind_rotate_tail_start(Form f, int groups, int count);
 
 // Key-switching table on the device: for t = 8 its words in FP16 pieces in

@@ -476,8 +476,8 @@ tfhe_gpu_status enqueue(tfhe_gpu_server* s, Tick& T) {
         const int groups = s->form == TFHE_GPU_SPLIT_FP32 && ctx->groups_per_cta[s->form] == 0
                                ? 15 : ctx->groups_per_cta[s->form];
         // As in a gate batch: when the blind rotation splits into full waves
-        // and a remainder wave on part of the SMs, the full waves' plain-gate
-        // key switch runs on the side stream during the remainder.
+        // and a remainder, the full waves' plain-gate key switch runs on the
+        // side stream beside the remainder, on the SMs that it leaves free.
         const int split = blind_rotate_tail_start((Form)s->form, groups, nb);
         const int k1 = std::min(split, nr);
         auto rotate = [&](int off, int cnt) -> cudaError_t {
